@@ -68,16 +68,16 @@ bool prefer_bulk(int M, int N, int K);
 int gemv_stream_supported(int M, int N, int K, int group, int bits, int lut_len, int x_dtype, int scale_dtype,
                           const void* x, const uint8_t* packed, const void* scales, int64_t packed_row_stride,
                           int64_t scale_row_stride, const void* zeros, int integer_grid, float grid_minimum);
-int launch_gemv_stream(const void* x, const uint8_t* packed, const void* scales, const float* lut, const void* bias,
-                       void* y, int M, int N, int K, int group, int bits, int lut_len, int64_t packed_row_stride,
-                       int64_t scale_row_stride, int integer_grid, float grid_minimum, int gated, cudaStream_t stream);
+int launch_gemv_stream(const void* x, const uint8_t* packed, const void* scales, const float* lut, const void* zeros,
+                       const void* bias, void* y, int M, int N, int K, int group, int bits, int lut_len, int x_dtype,
+                       int64_t packed_row_stride, int64_t scale_row_stride, int integer_grid, float grid_minimum,
+                       int gated, cudaStream_t stream);
 int gemv_stream_rotation_supported(int M, int N, int K, int group, int bits, int lut_len, int integer_grid,
                                    float grid_minimum, const void* signs);
 int launch_gemv_stream_rotated(const void* x, const uint8_t* packed, const void* scales, const float* lut,
                                const void* bias, void* y, int M, int N, int K, int group, int bits, int lut_len,
                                int64_t packed_row_stride, int64_t scale_row_stride, int integer_grid,
-                               float grid_minimum, int gated, const int8_t* signs, int rotate, int normalize,
-                               cudaStream_t stream);
+                               float grid_minimum, const int8_t* signs, int normalize, cudaStream_t stream);
 
 }  // namespace mkb
 
@@ -145,13 +145,13 @@ extern "C" int mkb_gemv_ws(const void* x, const uint8_t* packed, const void* sca
               "gemv: K=%d or group=%d splits a packing word of %d-bit codes", K, group, bits);
   MKB_REQUIRE(K > 0, MKB_E_UNSUPPORTED, "gemv: empty reduction");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const bool stream_ok = gemv_stream_supported(M, N, K, group, bits, lut_len, x_dtype, scale_dtype, x, packed, scales,
+  const bool stream_ok = (!gated || (x_dtype == MKB_F16 && zeros == nullptr && group >= 64)) && gemv_stream_supported(M, N, K, group, bits, lut_len, x_dtype, scale_dtype, x, packed, scales,
                                                packed_row_stride, scale_row_stride, zeros, integer_grid, grid_minimum);
-  if (kernel == MKB_GEMV_STREAM)
-    MKB_REQUIRE(stream_ok, MKB_E_UNSUPPORTED, "gemv: the streaming kernel does not cover these arguments");
+  if (kernel == MKB_GEMV_STREAM)   // by name: fp16 activations without offsets and one or two scales per 128 codes
+    MKB_REQUIRE(stream_ok && x_dtype == MKB_F16 && zeros == nullptr && group >= 64, MKB_E_UNSUPPORTED, "gemv: the streaming kernel does not cover these arguments");
   if (kernel == MKB_GEMV_STREAM || (kernel == MKB_GEMV_AUTO && stream_ok))
-    return launch_gemv_stream(x, packed, scales, lut, bias, y, M, N, K, group, bits, lut_len, packed_row_stride,
-                              scale_row_stride, integer_grid, grid_minimum, gated, s);
+    return launch_gemv_stream(x, packed, scales, lut, zeros, bias, y, M, N, K, group, bits, lut_len, x_dtype,
+                              packed_row_stride, scale_row_stride, integer_grid, grid_minimum, gated, s);
   const bool tiled_ok = gemv_tiled_supported(M, K, group, bits, x_dtype, scale_dtype, x, packed, packed_row_stride);
   const bool tmem_ok = workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) % 16) == 0 && lut_len == 16 &&
                        gemv_umma_supported(M, K, group, bits, x_dtype, scale_dtype, x, packed, packed_row_stride, zeros,
@@ -225,6 +225,6 @@ extern "C" int mkb_gemv_hadamard(const void* x, const int8_t* signs, const uint8
               "gemv_hadamard: needs a layer the streaming matvec covers, K a power of two of at least 512, "
               "M * K * 4 <= 65536 and 16-byte aligned signs");
   return launch_gemv_stream_rotated(x, packed, scales, lut, bias, y, M, N, K, group, bits, lut_len, packed_row_stride,
-                                    scale_row_stride, integer_grid, grid_minimum, 0, signs, 1, normalize,
+                                    scale_row_stride, integer_grid, grid_minimum, signs, normalize,
                                     static_cast<cudaStream_t>(stream));
 }

@@ -7,7 +7,7 @@
 // its word from bytes, expands the codes, forms w = lut[c] * scale (+ zero) in fp32 exactly like the
 // reference kernel does, and multiplies by up to eight activation rows.  Lane partials meet in a
 // shuffle tree; lane 0 adds the bias and stores in the activation dtype.
-#include "mkb_common.cuh"
+#include "scalar_row.cuh"
 
 namespace mkb {
 namespace {
@@ -36,32 +36,17 @@ __global__ void __launch_bounds__(kWarps * 32) gemv_scalar_kernel(ScalarArgs a) 
   const int row = blockIdx.x * kWarps + (threadIdx.x >> 5);
   if (row >= a.N) return;
 
-  const int wb = word_bytes(a.bits), wc = word_codes(a.bits);
-  const int words = a.K / wc;
-  const uint32_t mask = (1u << a.bits) - 1u;
-  const uint8_t* row_bytes = a.packed + int64_t(row) * a.packed_row_stride;
-  const bool has_zero = a.zeros != nullptr;
-
+  ScalarRow r{};
+  r.packed = a.packed + int64_t(row) * a.packed_row_stride;
+  r.scales = static_cast<const uint8_t*>(a.scales) + int64_t(row) * a.scale_row_stride * dtype_bytes(a.scale_dtype);
+  r.zeros = a.zeros == nullptr ? nullptr
+                               : static_cast<const uint8_t*>(a.zeros) + int64_t(row) * a.scale_row_stride * dtype_bytes(a.scale_dtype);
+  r.lut = lut_s; r.lut_len = 256;
+  r.K = a.K; r.group = a.group; r.bits = a.bits; r.x_dtype = a.x_dtype; r.scale_dtype = a.scale_dtype;
   float acc[MT];
 #pragma unroll
   for (int m = 0; m < MT; ++m) acc[m] = 0.f;
-
-  for (int w = lane; w < words; w += 32) {
-    uint64_t word = 0;
-    const uint8_t* p = row_bytes + int64_t(w) * wb;
-    for (int b = 0; b < wb; ++b) word |= uint64_t(__ldg(p + b)) << (8 * b);
-    const int k0 = w * wc;
-    const int64_t s_index = int64_t(row) * a.scale_row_stride + k0 / a.group;
-    const float scale = load_as_float(a.scales, s_index, a.scale_dtype);
-    const float zero = has_zero ? load_as_float(a.zeros, s_index, a.scale_dtype) : 0.f;
-    for (int c = 0; c < wc; ++c) {
-      const float value = lut_s[(word >> (c * a.bits)) & mask];
-      const float weight = has_zero ? reconstruct(value, scale, zero) : reconstruct(value, scale);
-#pragma unroll
-      for (int m = 0; m < MT; ++m)
-        if (m < a.M) acc[m] = fmaf(weight, load_as_float(a.x, int64_t(m) * a.K + k0 + c, a.x_dtype), acc[m]);
-    }
-  }
+  scalar_row_products<MT>(r, a.x, a.M, lane, acc);
 #pragma unroll
   for (int m = 0; m < MT; ++m)
     for (int offset = 16; offset; offset >>= 1) acc[m] += __shfl_xor_sync(0xffffffffu, acc[m], offset);

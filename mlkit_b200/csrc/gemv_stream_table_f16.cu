@@ -1,0 +1,8 @@
+// Instances of the streaming matvec: table codecs of 3 and 4 bits; f16 activations.
+#include "gemv_stream.cuh"
+
+namespace mkb {
+namespace stream {
+template int dispatch_table<X_F16>(const StreamArgs&, const StreamPlan&, cudaStream_t, int*);
+}  // namespace stream
+}  // namespace mkb
