@@ -242,6 +242,16 @@ int mkb_rtn_encode(const void* weight, const float* levels, uint8_t* packed, voi
                    int64_t N, int K, int group, int bits, int level_count, int integer_grid,
                    float grid_low, float grid_high, float reciprocal, int weight_dtype, void* stream);
 
+/* The same encoding with the scales as fp32 [N, ceil(K / group)] (the stored fp16 values, widened), with an offset per
+ * group in the same shape when `offsets` is not null (asymmetric formats: w = level * scale + offset), and with
+ * *nonfinite set to 1 when a weight is infinite or NaN (the caller clears it; the outputs are then meaningless).
+ * Covers groups of 8 to 256 codes (a power of two), K % 8 == 0 and a 16-byte aligned weight;
+ * everything else is MKB_E_UNSUPPORTED. */
+int mkb_rtn_encode_checked(const void* weight, const float* levels, uint8_t* packed, float* scales, float* offsets,
+                           uint8_t* codes_out, int* nonfinite, int64_t N, int K, int group, int bits, int level_count,
+                           int integer_grid, float grid_low, float grid_high, float reciprocal, int weight_dtype,
+                           void* stream);
+
 /*
  * Structured orthogonal transform of activation rows, fused:
  *   y[m,:] = (B kron H_pow2)(x[m,:] * signs), W = factor * pow2,

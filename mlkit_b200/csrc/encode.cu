@@ -6,8 +6,16 @@
 // reciprocal of the largest level magnitude, rounded to fp16 (clamped to [2^-24, 65504]); code =
 // round-half-even(w / scale) clamped to the grid for integer grids, the nearest level (a tie takes
 // the lower one) for codebooks; the division is IEEE binary32.
-// One warp encodes one group: a pass for the range, a pass for the codes (through shared memory),
-// then each lane assembles whole bytes of the stream.
+// Two kernels.
+//  * run kernel (groups of 8 to 256 codes, a power of two; rows of whole runs of eight codes): a lane owns eight
+//    consecutive weights, which are `bits` whole bytes of the stream.  The weights are read once, as 16-byte
+//    loads in their own type, and stay in registers; a group's range is a lane exchange; codes and stream leave as
+//    one store each.  Bound by memory: 3.5 bytes per bf16 weight at 4 bits (2 read, 1 + 0.5 written).  The IEEE
+//    division per weight would cost as much as the traffic, so an integer code is rounded from w * (1 / scale), and
+//    divided exactly only where that lies within the error bound of a rounding boundary.  An offset per group and a
+//    flag for infinities and NaNs are formed on the way.
+//  * group kernel (every other group): one warp per group, a pass for the range, a pass for the codes (through
+//    shared memory), then each lane assembles whole bytes of the stream.
 #include "mkb_common.cuh"
 
 namespace mkb {
@@ -25,6 +33,10 @@ struct EncodeArgs {
   int64_t rows;
   int width, group, groups, bits, level_count, integer, weight_dtype;
   float low, high, reciprocal;
+  // run kernel only
+  float* scales32;     // the stored scales widened
+  float* offsets32;    // asymmetric: the stored offsets widened
+  int* nonfinite;      // set to 1 when a weight is not finite
 };
 
 __device__ __forceinline__ int nearest_level(float x, const float* levels, int count) {
@@ -85,6 +97,195 @@ __global__ void __launch_bounds__(kEncodeWarps * 32) rtn_encode_kernel(const Enc
   }
 }
 
+// ---- run kernel ---------------------------------------------------------------------------------
+constexpr int kRunThreads = 256;
+constexpr int kRunsPerThread = 2;   // two 16-byte loads in flight per lane
+
+__device__ __forceinline__ void load_run8(const void* weight, int64_t at, int dtype, float (&w)[8]) {
+  if (dtype == MKB_F32) {
+    const float4* source = reinterpret_cast<const float4*>(static_cast<const float*>(weight) + at);
+    const float4 a = __ldcs(source), b = __ldcs(source + 1);
+    w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+    return;
+  }
+  const uint4 raw = __ldcs(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(weight) + at));
+  const uint32_t words[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 pair = dtype == MKB_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&words[i]))
+                                         : __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&words[i]));
+    w[2 * i] = pair.x;
+    w[2 * i + 1] = pair.y;
+  }
+}
+
+// round-half-even(w / scale), the division rounded to fp32 first.  The approximate quotient is within 2^-22 of that
+// one, relatively; unless a half-integer lies that close both round alike.  Quotients beyond the grid are clamped by
+// the caller whichever is taken.
+__device__ __forceinline__ float rounded_quotient(float w, float scale, float inverse, float margin) {
+  const float q = __fmul_rn(w, inverse), r = rintf(q);
+  if (fabsf(fabsf(q - r) - 0.5f) > margin) return r;
+  return rintf(__fdiv_rn(w, scale));
+}
+
+template <int BITS, bool INTEGER, bool ASYM>
+__global__ void __launch_bounds__(kRunThreads) rtn_encode_runs_kernel(const EncodeArgs a) {
+  __shared__ float level_s[256];
+  if constexpr (!INTEGER) {
+    for (int i = threadIdx.x; i < a.level_count; i += kRunThreads) level_s[i] = a.levels[i];
+    __syncthreads();
+  }
+  const uint32_t lanes_per_group = uint32_t(a.group) / 8, runs_per_row = uint32_t(a.groups) * lanes_per_group;
+  const uint32_t total = uint32_t(a.rows) * runs_per_row;
+  const uint32_t first = blockIdx.x * (kRunThreads * kRunsPerThread) + threadIdx.x;
+  float w[kRunsPerThread][8];
+  uint32_t row[kRunsPerThread], run[kRunsPerThread];
+  bool live[kRunsPerThread];
+#pragma unroll
+  for (int j = 0; j < kRunsPerThread; ++j) {
+    const uint32_t index = first + j * kRunThreads;
+    row[j] = index / runs_per_row;
+    run[j] = index - row[j] * runs_per_row;
+    live[j] = index < total && run[j] * 8 < uint32_t(a.width);    // the last group of a row may be short
+    if (live[j]) {
+      load_run8(a.weight, int64_t(row[j]) * a.width + run[j] * 8, a.weight_dtype, w[j]);
+    }
+  }
+  const float margin = (fmaxf(fabsf(a.low), fabsf(a.high)) + 2.f) * 4.76837158203125e-07f;   // 2^-21 of the largest quotient
+  bool bad = false;
+#pragma unroll
+  for (int j = 0; j < kRunsPerThread; ++j) {
+    float low = INFINITY, high = -INFINITY;
+    if (live[j]) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        bad |= !isfinite(w[j][e]);
+        low = fminf(low, w[j][e]);
+        high = fmaxf(high, w[j][e]);
+      }
+    }
+    for (uint32_t offset = lanes_per_group / 2; offset; offset >>= 1) {
+      low = fminf(low, __shfl_xor_sync(0xffffffffu, low, offset));
+      high = fmaxf(high, __shfl_xor_sync(0xffffffffu, high, offset));
+    }
+    const float range = ASYM ? __fsub_rn(high, low) : fmaxf(high, -low);
+    const float wide = __fmul_rn(fmaxf(range, 1e-12f), a.reciprocal);
+    const __half stored = __float2half_rn(fminf(fmaxf(wide, 5.9604644775390625e-08f), 65504.f));
+    const float scale = __half2float(stored);
+    float offset = 0.f;
+    if constexpr (ASYM) {
+      const float exact = __fsub_rn(low, __fmul_rn(a.low, wide));     // from the scale before it is stored
+      const float size = __half2float(__float2half_rn(fminf(fmaxf(fabsf(exact), 5.9604644775390625e-08f), 65504.f)));
+      offset = exact > 0.f ? size : exact < 0.f ? -size : 0.f;
+    }
+    if (!live[j]) continue;
+    const uint32_t group = run[j] / lanes_per_group;
+    if (run[j] - group * lanes_per_group == 0) {
+      const int64_t at = int64_t(row[j]) * a.groups + group;
+      if (a.scales != nullptr) a.scales[at] = stored;
+      if (a.scales32 != nullptr) a.scales32[at] = scale;
+      if constexpr (ASYM) a.offsets32[at] = offset;
+    }
+    const float inverse = __frcp_rn(scale);
+    uint32_t code[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float centred = ASYM ? __fsub_rn(w[j][e], offset) : w[j][e];
+      if constexpr (INTEGER)
+        code[e] = uint32_t(int(fminf(fmaxf(rounded_quotient(centred, scale, inverse, margin), a.low), a.high) - a.low));
+      else
+        code[e] = uint32_t(nearest_level(__fdiv_rn(centred, scale), level_s, a.level_count));
+    }
+    const int64_t at = int64_t(row[j]) * a.width + run[j] * 8;
+    if (a.codes != nullptr)
+      *reinterpret_cast<uint2*>(a.codes + at) = make_uint2(code[0] | code[1] << 8 | code[2] << 16 | code[3] << 24,
+                                                           code[4] | code[5] << 8 | code[6] << 16 | code[7] << 24);
+    uint64_t stream = 0;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) stream |= uint64_t(code[e]) << (e * BITS);
+    uint8_t* to = a.packed + at / 8 * BITS;
+    if constexpr (BITS == 8) *reinterpret_cast<uint2*>(to) = make_uint2(uint32_t(stream), uint32_t(stream >> 32));
+    else if constexpr (BITS == 4) *reinterpret_cast<uint32_t*>(to) = uint32_t(stream);
+    else if constexpr (BITS % 2 == 0) {
+#pragma unroll
+      for (int b = 0; b < BITS; b += 2) *reinterpret_cast<uint16_t*>(to + b) = uint16_t(stream >> (8 * b));
+    } else {
+#pragma unroll
+      for (int b = 0; b < BITS; ++b) to[b] = uint8_t(stream >> (8 * b));
+    }
+  }
+  if (bad && a.nonfinite != nullptr) *a.nonfinite = 1;
+}
+
+template <int BITS>
+void launch_runs(const EncodeArgs& a, unsigned blocks, cudaStream_t stream) {
+  const bool asym = a.offsets32 != nullptr;
+  if (a.integer) {
+    if (asym) rtn_encode_runs_kernel<BITS, true, true><<<blocks, kRunThreads, 0, stream>>>(a);
+    else rtn_encode_runs_kernel<BITS, true, false><<<blocks, kRunThreads, 0, stream>>>(a);
+  } else {
+    if (asym) rtn_encode_runs_kernel<BITS, false, true><<<blocks, kRunThreads, 0, stream>>>(a);
+    else rtn_encode_runs_kernel<BITS, false, false><<<blocks, kRunThreads, 0, stream>>>(a);
+  }
+}
+
+// Whether the run kernel covers a layout.
+bool runs_cover(const EncodeArgs& a) {
+  const auto aligned = [](const void* p, uintptr_t to) { return reinterpret_cast<uintptr_t>(p) % to == 0; };
+  const int lanes = a.group / 8;
+  return a.group % 8 == 0 && lanes <= 32 && (lanes & (lanes - 1)) == 0 && a.width % 8 == 0 && aligned(a.weight, 16) &&
+         aligned(a.packed, 8) && (a.codes == nullptr || aligned(a.codes, 8)) &&
+         a.rows * a.groups * lanes < (int64_t(1) << 31);
+}
+
+int encode(const EncodeArgs& a, cudaStream_t stream) {
+  if (runs_cover(a)) {
+    const int64_t total = a.rows * a.groups * (a.group / 8), per_block = kRunThreads * kRunsPerThread;
+    const unsigned blocks = unsigned((total + per_block - 1) / per_block);
+    switch (a.bits) {
+      case 1: launch_runs<1>(a, blocks, stream); break;
+      case 2: launch_runs<2>(a, blocks, stream); break;
+      case 3: launch_runs<3>(a, blocks, stream); break;
+      case 4: launch_runs<4>(a, blocks, stream); break;
+      case 5: launch_runs<5>(a, blocks, stream); break;
+      case 6: launch_runs<6>(a, blocks, stream); break;
+      case 7: launch_runs<7>(a, blocks, stream); break;
+      default: launch_runs<8>(a, blocks, stream); break;
+    }
+  } else {
+    MKB_REQUIRE(a.offsets32 == nullptr && a.scales32 == nullptr && a.nonfinite == nullptr, MKB_E_UNSUPPORTED,
+                "rtn_encode: offsets, wide scales and the finite check need groups of 8 to 256 codes (a power of two) and "
+                "rows of whole runs of eight");
+    const int64_t items = a.rows * a.groups;
+    const int64_t wanted = (items + kEncodeWarps - 1) / kEncodeWarps;
+    const int blocks = int(wanted < 148 * 16 ? wanted : 148 * 16);
+    rtn_encode_kernel<<<blocks, kEncodeWarps * 32, 0, stream>>>(a);
+  }
+  MKB_LAUNCH_CHECK("rtn_encode launch");
+  return MKB_OK;
+}
+
+int check_and_fill(EncodeArgs& a, const void* weight, const float* levels, uint8_t* packed, uint8_t* codes, int64_t N, int K,
+                   int group, int bits, int level_count, int integer_grid, float grid_low, float grid_high, float reciprocal,
+                   int weight_dtype) {
+  MKB_REQUIRE(N >= 0 && K >= 1 && group >= 1 && bits >= 1 && bits <= 8, MKB_E_ARGUMENT, "rtn_encode: bad shape");
+  MKB_REQUIRE(level_count >= 1 && level_count <= (1 << bits), MKB_E_ARGUMENT,
+              "rtn_encode: %d levels do not fit %d-bit codes", level_count, bits);
+  MKB_REQUIRE(weight_dtype >= MKB_F16 && weight_dtype <= MKB_F32, MKB_E_ARGUMENT, "rtn_encode: unknown dtype");
+  MKB_REQUIRE(grid_high >= grid_low && reciprocal > 0.f, MKB_E_ARGUMENT, "rtn_encode: bad grid range");
+  if (N == 0) return MKB_OK;
+  MKB_REQUIRE(weight && levels && packed, MKB_E_ARGUMENT, "rtn_encode: null pointer");
+  if (group > K) group = K;
+  MKB_REQUIRE(group <= kMaxGroup, MKB_E_UNSUPPORTED, "rtn_encode: groups of more than %d codes", kMaxGroup);
+  MKB_REQUIRE((int64_t(group) * bits) % 8 == 0 && (int64_t(K) * bits) % 8 == 0, MKB_E_UNSUPPORTED,
+              "rtn_encode: a group or a row of %d-bit codes does not end on a byte", bits);
+  a.weight = weight; a.levels = levels; a.packed = packed; a.codes = codes;
+  a.rows = N; a.width = K; a.group = group; a.groups = (K + group - 1) / group; a.bits = bits;
+  a.level_count = level_count; a.integer = integer_grid; a.weight_dtype = weight_dtype;
+  a.low = grid_low; a.high = grid_high; a.reciprocal = reciprocal;
+  return MKB_OK;
+}
+
 }  // namespace
 }  // namespace mkb
 
@@ -92,26 +293,28 @@ extern "C" int mkb_rtn_encode(const void* weight, const float* levels, uint8_t* 
                               int64_t N, int K, int group, int bits, int level_count, int integer_grid,
                               float grid_low, float grid_high, float reciprocal, int weight_dtype, void* stream) {
   using namespace mkb;
-  MKB_REQUIRE(N >= 0 && K >= 1 && group >= 1 && bits >= 1 && bits <= 8, MKB_E_ARGUMENT, "rtn_encode: bad shape");
-  MKB_REQUIRE(level_count >= 1 && level_count <= (1 << bits), MKB_E_ARGUMENT,
-              "rtn_encode: %d levels do not fit %d-bit codes", level_count, bits);
-  MKB_REQUIRE(weight_dtype >= MKB_F16 && weight_dtype <= MKB_F32, MKB_E_ARGUMENT, "rtn_encode: unknown dtype");
-  MKB_REQUIRE(grid_high >= grid_low && reciprocal > 0.f, MKB_E_ARGUMENT, "rtn_encode: bad grid range");
-  if (N == 0) return MKB_OK;
-  MKB_REQUIRE(weight && levels && packed && scales, MKB_E_ARGUMENT, "rtn_encode: null pointer");
-  if (group > K) group = K;
-  MKB_REQUIRE(group <= kMaxGroup, MKB_E_UNSUPPORTED, "rtn_encode: groups of more than %d codes", kMaxGroup);
-  MKB_REQUIRE((int64_t(group) * bits) % 8 == 0 && (int64_t(K) * bits) % 8 == 0, MKB_E_UNSUPPORTED,
-              "rtn_encode: a group or a row of %d-bit codes does not end on a byte", bits);
   EncodeArgs a{};
-  a.weight = weight; a.levels = levels; a.packed = packed; a.scales = static_cast<__half*>(scales); a.codes = codes;
-  a.rows = N; a.width = K; a.group = group; a.groups = (K + group - 1) / group; a.bits = bits;
-  a.level_count = level_count; a.integer = integer_grid; a.weight_dtype = weight_dtype;
-  a.low = grid_low; a.high = grid_high; a.reciprocal = reciprocal;
-  const int64_t items = N * a.groups;
-  const int64_t wanted = (items + kEncodeWarps - 1) / kEncodeWarps;
-  const int blocks = int(wanted < 148 * 16 ? wanted : 148 * 16);
-  rtn_encode_kernel<<<blocks, kEncodeWarps * 32, 0, static_cast<cudaStream_t>(stream)>>>(a);
-  MKB_LAUNCH_CHECK("rtn_encode launch");
-  return MKB_OK;
+  const int status = check_and_fill(a, weight, levels, packed, codes, N, K, group, bits, level_count, integer_grid, grid_low,
+                                    grid_high, reciprocal, weight_dtype);
+  if (status != MKB_OK || N == 0) return status;
+  MKB_REQUIRE(scales != nullptr, MKB_E_ARGUMENT, "rtn_encode: null pointer");
+  a.scales = static_cast<__half*>(scales);
+  return encode(a, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int mkb_rtn_encode_checked(const void* weight, const float* levels, uint8_t* packed, float* scales, float* offsets,
+                                      uint8_t* codes, int* nonfinite, int64_t N, int K, int group, int bits,
+                                      int level_count, int integer_grid, float grid_low, float grid_high,
+                                      float reciprocal, int weight_dtype, void* stream) {
+  using namespace mkb;
+  EncodeArgs a{};
+  const int status = check_and_fill(a, weight, levels, packed, codes, N, K, group, bits, level_count, integer_grid, grid_low,
+                                    grid_high, reciprocal, weight_dtype);
+  if (status != MKB_OK || N == 0) return status;
+  MKB_REQUIRE(scales != nullptr && nonfinite != nullptr, MKB_E_ARGUMENT, "rtn_encode_checked: null pointer");
+  a.scales32 = scales; a.offsets32 = offsets; a.nonfinite = nonfinite;
+  MKB_REQUIRE(runs_cover(a), MKB_E_UNSUPPORTED,
+              "rtn_encode_checked: needs groups of 8 to 256 codes (a power of two), rows of whole runs of eight codes and a "
+              "16-byte aligned weight");
+  return encode(a, static_cast<cudaStream_t>(stream));
 }

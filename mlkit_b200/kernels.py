@@ -328,6 +328,36 @@ def rtn_encode(weight: Tensor, levels: Tensor, *, group: int, bits: int, integer
     return packed, scales, unpacked
 
 
+def checked_encode_supported(weight: Tensor, group: int) -> bool:
+    """Whether ``rtn_encode_checked`` covers the layout (the C entry point checks the same): groups of 8 to 256 codes,
+    a power of two, in rows of whole runs of eight."""
+    rows, width = weight.shape
+    group = min(group, width)
+    return (weight.dtype in DTYPE_TAGS and weight.is_contiguous() and weight.data_ptr() % 16 == 0 and width % 8 == 0
+            and 8 <= group <= 256 and group & (group - 1) == 0 and 0 < rows * (width + group) < 1 << 34)
+
+
+def rtn_encode_checked(weight: Tensor, levels: Tensor, *, group: int, bits: int, integer_grid: bool, low: float, high: float,
+                       reciprocal: float, asym: bool) -> tuple[Tensor, Tensor, Tensor | None, Tensor, Tensor]:
+    """``rtn_encode`` of a weight in its own type, with offsets when ``asym``: returns ``(packed uint8, scales fp32,
+    offsets fp32 or None, codes uint8, nonfinite int32 [1])``.  ``nonfinite`` is 1 when a weight is not finite."""
+    device = _require_cuda(weight, levels)
+    rows, width = weight.shape
+    group = min(group, width)
+    packed = torch.empty(rows * width * bits // 8, dtype=torch.uint8, device=device)
+    scales = torch.empty((rows, -(-width // group)), dtype=torch.float32, device=device)
+    offsets = torch.empty_like(scales) if asym else None
+    codes = torch.empty((rows, width), dtype=torch.uint8, device=device)
+    nonfinite = torch.zeros(1, dtype=torch.int32, device=device)
+    with torch.cuda.device(device):
+        status = _native.library().mkb_rtn_encode_checked(
+            weight.data_ptr(), levels.data_ptr(), packed.data_ptr(), scales.data_ptr(), _pointer(offsets), codes.data_ptr(),
+            nonfinite.data_ptr(), rows, width, group, bits, levels.numel(), int(integer_grid), float(low), float(high),
+            float(reciprocal), _tag(weight.dtype, "weight"), _stream(device))
+    _native.check(status, "rtn_encode_checked")
+    return packed, scales, offsets, codes, nonfinite
+
+
 def dequantize_rows(packed: Tensor, scales: Tensor, values: Tensor, zeros: Tensor | None, rows: Tensor, *,
                     shape: tuple[int, int], group: int, bits: int, dtype: torch.dtype) -> Tensor:
     """Reconstruct the listed rows only: ``out[i] = weight[rows[i]]``."""

@@ -419,11 +419,32 @@ class Scaled:
     def __call__(self, w: Tensor, ctx: Ctx | None = None) -> Q:
         if w.ndim != 2 or not w.is_floating_point():
             raise ValueError("scaled requires a finite floating-point weight matrix")
-        weight = w.float()
-        rows, width = weight.shape
+        rows, width = w.shape
         group = width if self.group is None else min(self.group, width)
-        levels = self.grid.values.to(weight.device).contiguous()
+        levels = self.grid.values.to(w.device).contiguous()
         bits = self.grid.bits
+        if w.is_cuda and self.scale == "absmax" and self.scale_fmt == "fp16" and bits <= 8:
+            # one launch on the device, from the weight in its own type: the arithmetic of the tensor route below,
+            # operation for operation
+            from mlkit_b200 import kernels
+
+            differentiable = self.asym and w.requires_grad and torch.is_grad_enabled()   # of the tensor route only
+            if not differentiable and kernels.checked_encode_supported(w, group):
+                stream, scales, zero, codes, nonfinite = kernels.rtn_encode_checked(
+                    w, levels, group=group, bits=bits, integer_grid=self.grid.integer, low=self._low, high=self._high,
+                    reciprocal=self._reciprocal, asym=self.asym)
+                if nonfinite.item():
+                    raise ValueError("scaled requires a finite floating-point weight matrix")
+                encoded = Q(
+                    bits=bits * w.numel() + scales.numel() * (32 if self.asym else 16), codes=codes,
+                    params={"scales": scales, "values": levels, "group": group, "offset": 0, "zero": zero},
+                    decode=decode_scaled, codec="scaled",
+                    metadata={"code_bits": bits, "scale_fmt": self.scale_fmt,
+                              "trainable": ["scales"] + (["zero"] if self.asym else [])},
+                )
+                encoded._stream = (stream, codes, _version_of(codes), bits)
+                return encoded
+        weight = w.float()
         if (weight.is_cuda and self.scale == "absmax" and not self.asym and self.scale_fmt == "fp16" and bits <= 8
                 and group <= 1024 and (group * bits) % 8 == 0 and (width * bits) % 8 == 0 and rows > 0):
             # one launch on the device: the same arithmetic, operation for operation (mkb_rtn_encode)
