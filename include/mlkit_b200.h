@@ -244,7 +244,8 @@ int mkb_rtn_encode(const void* weight, const float* levels, uint8_t* packed, voi
 
 /* The same encoding with the scales as fp32 [N, ceil(K / group)] (the stored fp16 values, widened), with an offset per
  * group in the same shape when `offsets` is not null (asymmetric formats: w = level * scale + offset), and with
- * *nonfinite set to 1 when a weight is infinite or NaN (the caller clears it; the outputs are then meaningless).
+ * *nonfinite (device) set to 0, or to 1 when a weight is infinite or NaN (the outputs are then meaningless).
+ * `levels` may be null for integer grids.
  * Covers groups of 8 to 256 codes (a power of two), K % 8 == 0 and a 16-byte aligned weight;
  * everything else is MKB_E_UNSUPPORTED. */
 int mkb_rtn_encode_checked(const void* weight, const float* levels, uint8_t* packed, float* scales, float* offsets,

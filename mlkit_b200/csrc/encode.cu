@@ -11,8 +11,8 @@
 //    consecutive weights, which are `bits` whole bytes of the stream.  The weights are read once, as 16-byte
 //    loads in their own type, and stay in registers; a group's range is a lane exchange; codes and stream leave as
 //    one store each.  Bound by memory: 3.5 bytes per bf16 weight at 4 bits (2 read, 1 + 0.5 written).  The IEEE
-//    division per weight would cost as much as the traffic, so an integer code is rounded from w * (1 / scale), and
-//    divided exactly only where that lies within the error bound of a rounding boundary.  An offset per group and a
+//    division per weight and the conversions to integers would cost more than the traffic, so the quotient is formed
+//    from the group's reciprocal (three operations, same rounding) and rounded to an integer by an addition.  An offset per group and a
 //    flag for infinities and NaNs are formed on the way.
 //  * group kernel (every other group): one warp per group, a pass for the range, a pass for the codes (through
 //    shared memory), then each lane assembles whole bytes of the stream.
@@ -37,6 +37,9 @@ struct EncodeArgs {
   float* scales32;     // the stored scales widened
   float* offsets32;    // asymmetric: the stored offsets widened
   int* nonfinite;      // set to 1 when a weight is not finite
+  int lane_shift;      // log2(group / 8): lanes of a group
+  uint32_t row_magic;  // index / (groups << lane_shift) = (umulhi(magic, index) + index) >> shift, for index < 2^31
+  int row_shift;
 };
 
 __device__ __forceinline__ int nearest_level(float x, const float* levels, int count) {
@@ -100,32 +103,53 @@ __global__ void __launch_bounds__(kEncodeWarps * 32) rtn_encode_kernel(const Enc
 // ---- run kernel ---------------------------------------------------------------------------------
 constexpr int kRunThreads = 256;
 constexpr int kRunsPerThread = 2;   // two 16-byte loads in flight per lane
+constexpr float kRoundMagic = 12582912.f;           // 1.5 * 2^23: adding it rounds |x| < 2^22 half to even
+constexpr uint32_t kRoundMagicBits = 0x4b400000u;   // and leaves the integer in the low bits
 
-__device__ __forceinline__ void load_run8(const void* weight, int64_t at, int dtype, float (&w)[8]) {
+// eight weights and the bits of their largest magnitude (a NaN's exceed an infinity's)
+__device__ __forceinline__ void load_run8(const void* weight, int64_t at, int dtype, float (&w)[8], uint32_t& largest) {
   if (dtype == MKB_F32) {
-    const float4* source = reinterpret_cast<const float4*>(static_cast<const float*>(weight) + at);
-    const float4 a = __ldcs(source), b = __ldcs(source + 1);
-    w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+    const uint4* source = reinterpret_cast<const uint4*>(static_cast<const float*>(weight) + at);
+    const uint4 a = __ldcs(source), b = __ldcs(source + 1);
+    const uint32_t bits[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      w[e] = __uint_as_float(bits[e]);
+      largest = max(largest, bits[e] & 0x7fffffffu);
+    }
     return;
   }
   const uint4 raw = __ldcs(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(weight) + at));
   const uint32_t words[4] = {raw.x, raw.y, raw.z, raw.w};
+  uint32_t pair = 0;   // of the magnitudes, both halves of a word at once
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 pair = dtype == MKB_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&words[i]))
-                                         : __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&words[i]));
-    w[2 * i] = pair.x;
-    w[2 * i + 1] = pair.y;
+  for (int i = 0; i < 4; ++i) pair = __vmaxu2(pair, words[i] & 0x7fff7fffu);
+  const uint32_t half = max(pair & 0xffffu, pair >> 16);
+  if (dtype == MKB_F16) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 two = __half22float2(*reinterpret_cast<const __half2*>(&words[i]));
+      w[2 * i] = two.x;
+      w[2 * i + 1] = two.y;
+    }
+    largest = half >= 0x7c00u ? 0x7f800000u : __float_as_uint(__half2float(__ushort_as_half((unsigned short)half)));
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      w[2 * i] = __uint_as_float(words[i] << 16);
+      w[2 * i + 1] = __uint_as_float(words[i] & 0xffff0000u);
+    }
+    largest = half << 16;
   }
 }
 
-// round-half-even(w / scale), the division rounded to fp32 first.  The approximate quotient is within 2^-22 of that
-// one, relatively; unless a half-integer lies that close both round alike.  Quotients beyond the grid are clamped by
-// the caller whichever is taken.
-__device__ __forceinline__ float rounded_quotient(float w, float scale, float inverse, float margin) {
-  const float q = __fmul_rn(w, inverse), r = rintf(q);
-  if (fabsf(fabsf(q - r) - 0.5f) > margin) return r;
-  return rintf(__fdiv_rn(w, scale));
+// w / scale rounded to fp32, by Markstein's correction of an approximate quotient: the remainder w - q * scale is
+// exact, and q plus remainder times reciprocal misses the quotient by 2^-46 of it before its one rounding.  A stored
+// scale has eleven significant bits, so no quotient lies within 2^-36 of a point where the rounding would change:
+// the result is the IEEE division's.  (Where the remainder underflows the quotient rounds to zero codes anyway.)
+__device__ __forceinline__ float quotient(float w, float scale, float inverse) {
+  const float q = __fmul_rn(w, inverse);
+  return __fmaf_rn(__fmaf_rn(-q, scale, w), inverse, q);
 }
 
 template <int BITS, bool INTEGER, bool ASYM>
@@ -135,40 +159,45 @@ __global__ void __launch_bounds__(kRunThreads) rtn_encode_runs_kernel(const Enco
     for (int i = threadIdx.x; i < a.level_count; i += kRunThreads) level_s[i] = a.levels[i];
     __syncthreads();
   }
-  const uint32_t lanes_per_group = uint32_t(a.group) / 8, runs_per_row = uint32_t(a.groups) * lanes_per_group;
+  const uint32_t lanes_per_group = 1u << a.lane_shift, runs_per_row = uint32_t(a.groups) << a.lane_shift;
   const uint32_t total = uint32_t(a.rows) * runs_per_row;
   const uint32_t first = blockIdx.x * (kRunThreads * kRunsPerThread) + threadIdx.x;
   float w[kRunsPerThread][8];
-  uint32_t row[kRunsPerThread], run[kRunsPerThread];
+  uint32_t row[kRunsPerThread], run[kRunsPerThread], largest[kRunsPerThread];
   bool live[kRunsPerThread];
 #pragma unroll
   for (int j = 0; j < kRunsPerThread; ++j) {
     const uint32_t index = first + j * kRunThreads;
-    row[j] = index / runs_per_row;
+    row[j] = (__umulhi(a.row_magic, index) + index) >> a.row_shift;   // index / runs_per_row
     run[j] = index - row[j] * runs_per_row;
     live[j] = index < total && run[j] * 8 < uint32_t(a.width);    // the last group of a row may be short
-    if (live[j]) {
-      load_run8(a.weight, int64_t(row[j]) * a.width + run[j] * 8, a.weight_dtype, w[j]);
-    }
+    largest[j] = 0;
+    if (live[j]) load_run8(a.weight, int64_t(row[j]) * a.width + run[j] * 8, a.weight_dtype, w[j], largest[j]);
   }
-  const float margin = (fmaxf(fabsf(a.low), fabsf(a.high)) + 2.f) * 4.76837158203125e-07f;   // 2^-21 of the largest quotient
   bool bad = false;
 #pragma unroll
   for (int j = 0; j < kRunsPerThread; ++j) {
-    float low = INFINITY, high = -INFINITY;
-    if (live[j]) {
+    bad |= largest[j] >= 0x7f800000u;
+    float low = INFINITY, range;
+    if constexpr (ASYM) {
+      float high = -INFINITY;
+      if (live[j]) {
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        bad |= !isfinite(w[j][e]);
-        low = fminf(low, w[j][e]);
-        high = fmaxf(high, w[j][e]);
+        for (int e = 0; e < 8; ++e) {
+          low = fminf(low, w[j][e]);
+          high = fmaxf(high, w[j][e]);
+        }
       }
+      for (uint32_t offset = lanes_per_group / 2; offset; offset >>= 1) {
+        low = fminf(low, __shfl_xor_sync(0xffffffffu, low, offset));
+        high = fmaxf(high, __shfl_xor_sync(0xffffffffu, high, offset));
+      }
+      range = __fsub_rn(high, low);
+    } else {
+      for (uint32_t offset = lanes_per_group / 2; offset; offset >>= 1)
+        largest[j] = max(largest[j], __shfl_xor_sync(0xffffffffu, largest[j], offset));
+      range = __uint_as_float(largest[j]);
     }
-    for (uint32_t offset = lanes_per_group / 2; offset; offset >>= 1) {
-      low = fminf(low, __shfl_xor_sync(0xffffffffu, low, offset));
-      high = fmaxf(high, __shfl_xor_sync(0xffffffffu, high, offset));
-    }
-    const float range = ASYM ? __fsub_rn(high, low) : fmaxf(high, -low);
     const float wide = __fmul_rn(fmaxf(range, 1e-12f), a.reciprocal);
     const __half stored = __float2half_rn(fminf(fmaxf(wide, 5.9604644775390625e-08f), 65504.f));
     const float scale = __half2float(stored);
@@ -179,39 +208,53 @@ __global__ void __launch_bounds__(kRunThreads) rtn_encode_runs_kernel(const Enco
       offset = exact > 0.f ? size : exact < 0.f ? -size : 0.f;
     }
     if (!live[j]) continue;
-    const uint32_t group = run[j] / lanes_per_group;
-    if (run[j] - group * lanes_per_group == 0) {
-      const int64_t at = int64_t(row[j]) * a.groups + group;
+    if ((run[j] & (lanes_per_group - 1)) == 0) {
+      const int64_t at = int64_t(row[j]) * a.groups + (run[j] >> a.lane_shift);
       if (a.scales != nullptr) a.scales[at] = stored;
       if (a.scales32 != nullptr) a.scales32[at] = scale;
       if constexpr (ASYM) a.offsets32[at] = offset;
     }
-    const float inverse = __frcp_rn(scale);
+    // codes as the low bits of `code` once `base` is taken away (of all of them at once, modulo the word)
     uint32_t code[8];
+    constexpr uint32_t base = INTEGER ? kRoundMagicBits : 0u;
+    const float inverse = __frcp_rn(scale);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      const float centred = ASYM ? __fsub_rn(w[j][e], offset) : w[j][e];
-      if constexpr (INTEGER)
-        code[e] = uint32_t(int(fminf(fmaxf(rounded_quotient(centred, scale, inverse, margin), a.low), a.high) - a.low));
-      else
-        code[e] = uint32_t(nearest_level(__fdiv_rn(centred, scale), level_s, a.level_count));
+      const float q = quotient(ASYM ? __fsub_rn(w[j][e], offset) : w[j][e], scale, inverse);
+      if constexpr (INTEGER) code[e] = __float_as_uint(__fadd_rn(fminf(fmaxf(q, a.low), a.high), kRoundMagic));
+      else code[e] = uint32_t(nearest_level(q, level_s, a.level_count));
     }
+    const uint32_t shift = INTEGER ? base + uint32_t(int(a.low)) : 0u;   // what a code of zero looks like
     const int64_t at = int64_t(row[j]) * a.width + run[j] * 8;
-    if (a.codes != nullptr)
-      *reinterpret_cast<uint2*>(a.codes + at) = make_uint2(code[0] | code[1] << 8 | code[2] << 16 | code[3] << 24,
-                                                           code[4] | code[5] << 8 | code[6] << 16 | code[7] << 24);
-    uint64_t stream = 0;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) stream |= uint64_t(code[e]) << (e * BITS);
+    if (a.codes != nullptr) {
+      const uint32_t off = shift * 0x01010101u;
+      *reinterpret_cast<uint2*>(a.codes + at) =
+          make_uint2(code[0] + (code[1] << 8) + (code[2] << 16) + (code[3] << 24) - off,
+                     code[4] + (code[5] << 8) + (code[6] << 16) + (code[7] << 24) - off);
+    }
     uint8_t* to = a.packed + at / 8 * BITS;
-    if constexpr (BITS == 8) *reinterpret_cast<uint2*>(to) = make_uint2(uint32_t(stream), uint32_t(stream >> 32));
-    else if constexpr (BITS == 4) *reinterpret_cast<uint32_t*>(to) = uint32_t(stream);
-    else if constexpr (BITS % 2 == 0) {
+    if constexpr (BITS <= 4) {
+      uint32_t stream = 0;
 #pragma unroll
-      for (int b = 0; b < BITS; b += 2) *reinterpret_cast<uint16_t*>(to + b) = uint16_t(stream >> (8 * b));
+      for (int e = 0; e < 8; ++e) stream += (code[e] - shift) << (e * BITS);
+      if constexpr (BITS == 4) *reinterpret_cast<uint32_t*>(to) = stream;
+      else if constexpr (BITS == 2) *reinterpret_cast<uint16_t*>(to) = uint16_t(stream);
+      else {
+#pragma unroll
+        for (int b = 0; b < BITS; ++b) to[b] = uint8_t(stream >> (8 * b));
+      }
     } else {
+      uint64_t stream = 0;
 #pragma unroll
-      for (int b = 0; b < BITS; ++b) to[b] = uint8_t(stream >> (8 * b));
+      for (int e = 0; e < 8; ++e) stream |= uint64_t(code[e] - shift) << (e * BITS);
+      if constexpr (BITS == 8) *reinterpret_cast<uint2*>(to) = make_uint2(uint32_t(stream), uint32_t(stream >> 32));
+      else if constexpr (BITS == 6) {
+#pragma unroll
+        for (int b = 0; b < BITS; b += 2) *reinterpret_cast<uint16_t*>(to + b) = uint16_t(stream >> (8 * b));
+      } else {
+#pragma unroll
+        for (int b = 0; b < BITS; ++b) to[b] = uint8_t(stream >> (8 * b));
+      }
     }
   }
   if (bad && a.nonfinite != nullptr) *a.nonfinite = 1;
@@ -238,8 +281,13 @@ bool runs_cover(const EncodeArgs& a) {
          a.rows * a.groups * lanes < (int64_t(1) << 31);
 }
 
-int encode(const EncodeArgs& a, cudaStream_t stream) {
+int encode(EncodeArgs a, cudaStream_t stream) {
   if (runs_cover(a)) {
+    while ((8 << a.lane_shift) < a.group) ++a.lane_shift;
+    // the round-up method of dividing by an invariant: 2^shift is the next power of two from the divisor
+    const uint32_t divisor = uint32_t(a.groups) << a.lane_shift;
+    while ((uint64_t(1) << a.row_shift) < divisor) ++a.row_shift;
+    a.row_magic = uint32_t((((uint64_t(1) << a.row_shift) - divisor) << 32) / divisor + 1);
     const int64_t total = a.rows * a.groups * (a.group / 8), per_block = kRunThreads * kRunsPerThread;
     const unsigned blocks = unsigned((total + per_block - 1) / per_block);
     switch (a.bits) {
@@ -274,7 +322,7 @@ int check_and_fill(EncodeArgs& a, const void* weight, const float* levels, uint8
   MKB_REQUIRE(weight_dtype >= MKB_F16 && weight_dtype <= MKB_F32, MKB_E_ARGUMENT, "rtn_encode: unknown dtype");
   MKB_REQUIRE(grid_high >= grid_low && reciprocal > 0.f, MKB_E_ARGUMENT, "rtn_encode: bad grid range");
   if (N == 0) return MKB_OK;
-  MKB_REQUIRE(weight && levels && packed, MKB_E_ARGUMENT, "rtn_encode: null pointer");
+  MKB_REQUIRE(weight && packed, MKB_E_ARGUMENT, "rtn_encode: null pointer");
   if (group > K) group = K;
   MKB_REQUIRE(group <= kMaxGroup, MKB_E_UNSUPPORTED, "rtn_encode: groups of more than %d codes", kMaxGroup);
   MKB_REQUIRE((int64_t(group) * bits) % 8 == 0 && (int64_t(K) * bits) % 8 == 0, MKB_E_UNSUPPORTED,
@@ -297,7 +345,7 @@ extern "C" int mkb_rtn_encode(const void* weight, const float* levels, uint8_t* 
   const int status = check_and_fill(a, weight, levels, packed, codes, N, K, group, bits, level_count, integer_grid, grid_low,
                                     grid_high, reciprocal, weight_dtype);
   if (status != MKB_OK || N == 0) return status;
-  MKB_REQUIRE(scales != nullptr, MKB_E_ARGUMENT, "rtn_encode: null pointer");
+  MKB_REQUIRE(scales != nullptr && levels != nullptr, MKB_E_ARGUMENT, "rtn_encode: null pointer");
   a.scales = static_cast<__half*>(scales);
   return encode(a, static_cast<cudaStream_t>(stream));
 }
@@ -311,10 +359,12 @@ extern "C" int mkb_rtn_encode_checked(const void* weight, const float* levels, u
   const int status = check_and_fill(a, weight, levels, packed, codes, N, K, group, bits, level_count, integer_grid, grid_low,
                                     grid_high, reciprocal, weight_dtype);
   if (status != MKB_OK || N == 0) return status;
-  MKB_REQUIRE(scales != nullptr && nonfinite != nullptr, MKB_E_ARGUMENT, "rtn_encode_checked: null pointer");
+  MKB_REQUIRE(scales != nullptr && nonfinite != nullptr && (levels != nullptr || integer_grid), MKB_E_ARGUMENT, "rtn_encode_checked: null pointer");
   a.scales32 = scales; a.offsets32 = offsets; a.nonfinite = nonfinite;
   MKB_REQUIRE(runs_cover(a), MKB_E_UNSUPPORTED,
               "rtn_encode_checked: needs groups of 8 to 256 codes (a power of two), rows of whole runs of eight codes and a "
               "16-byte aligned weight");
+  const cudaError_t cleared = cudaMemsetAsync(nonfinite, 0, sizeof(int), static_cast<cudaStream_t>(stream));
+  if (cleared != cudaSuccess) return cuda_fail(cleared, "rtn_encode_checked: clearing the flag");
   return encode(a, static_cast<cudaStream_t>(stream));
 }

@@ -337,10 +337,11 @@ def checked_encode_supported(weight: Tensor, group: int) -> bool:
             and 8 <= group <= 256 and group & (group - 1) == 0 and 0 < rows * (width + group) < 1 << 34)
 
 
-def rtn_encode_checked(weight: Tensor, levels: Tensor, *, group: int, bits: int, integer_grid: bool, low: float, high: float,
+def rtn_encode_checked(weight: Tensor, levels: Tensor | None, *, group: int, bits: int, integer_grid: bool, low: float, high: float,
                        reciprocal: float, asym: bool) -> tuple[Tensor, Tensor, Tensor | None, Tensor, Tensor]:
     """``rtn_encode`` of a weight in its own type, with offsets when ``asym``: returns ``(packed uint8, scales fp32,
-    offsets fp32 or None, codes uint8, nonfinite int32 [1])``.  ``nonfinite`` is 1 when a weight is not finite."""
+    offsets fp32 or None, codes uint8, nonfinite int32 [1])``.  ``nonfinite`` is 1 when a weight is not finite.
+    Integer grids need no ``levels``."""
     device = _require_cuda(weight, levels)
     rows, width = weight.shape
     group = min(group, width)
@@ -348,11 +349,11 @@ def rtn_encode_checked(weight: Tensor, levels: Tensor, *, group: int, bits: int,
     scales = torch.empty((rows, -(-width // group)), dtype=torch.float32, device=device)
     offsets = torch.empty_like(scales) if asym else None
     codes = torch.empty((rows, width), dtype=torch.uint8, device=device)
-    nonfinite = torch.zeros(1, dtype=torch.int32, device=device)
+    nonfinite = torch.empty(1, dtype=torch.int32, device=device)
     with torch.cuda.device(device):
         status = _native.library().mkb_rtn_encode_checked(
-            weight.data_ptr(), levels.data_ptr(), packed.data_ptr(), scales.data_ptr(), _pointer(offsets), codes.data_ptr(),
-            nonfinite.data_ptr(), rows, width, group, bits, levels.numel(), int(integer_grid), float(low), float(high),
+            weight.data_ptr(), _pointer(levels), packed.data_ptr(), scales.data_ptr(), _pointer(offsets), codes.data_ptr(),
+            nonfinite.data_ptr(), rows, width, group, bits, 1 if levels is None else levels.numel(), int(integer_grid), float(low), float(high),
             float(reciprocal), _tag(weight.dtype, "weight"), _stream(device))
     _native.check(status, "rtn_encode_checked")
     return packed, scales, offsets, codes, nonfinite

@@ -421,7 +421,6 @@ class Scaled:
             raise ValueError("scaled requires a finite floating-point weight matrix")
         rows, width = w.shape
         group = width if self.group is None else min(self.group, width)
-        levels = self.grid.values.to(w.device).contiguous()
         bits = self.grid.bits
         if w.is_cuda and self.scale == "absmax" and self.scale_fmt == "fp16" and bits <= 8:
             # one launch on the device, from the weight in its own type: the arithmetic of the tensor route below,
@@ -430,11 +429,13 @@ class Scaled:
 
             differentiable = self.asym and w.requires_grad and torch.is_grad_enabled()   # of the tensor route only
             if not differentiable and kernels.checked_encode_supported(w, group):
+                # an integer grid's levels are copied to the device behind the launch, which does not read them
+                levels = None if self.grid.integer else self.grid.values.to(w.device).contiguous()
                 stream, scales, zero, codes, nonfinite = kernels.rtn_encode_checked(
                     w, levels, group=group, bits=bits, integer_grid=self.grid.integer, low=self._low, high=self._high,
                     reciprocal=self._reciprocal, asym=self.asym)
-                if nonfinite.item():
-                    raise ValueError("scaled requires a finite floating-point weight matrix")
+                if levels is None:
+                    levels = self.grid.values.to(w.device).contiguous()
                 encoded = Q(
                     bits=bits * w.numel() + scales.numel() * (32 if self.asym else 16), codes=codes,
                     params={"scales": scales, "values": levels, "group": group, "offset": 0, "zero": zero},
@@ -443,7 +444,10 @@ class Scaled:
                               "trainable": ["scales"] + (["zero"] if self.asym else [])},
                 )
                 encoded._stream = (stream, codes, _version_of(codes), bits)
+                if nonfinite.item():
+                    raise ValueError("scaled requires a finite floating-point weight matrix")
                 return encoded
+        levels = self.grid.values.to(w.device).contiguous()
         weight = w.float()
         if (weight.is_cuda and self.scale == "absmax" and not self.asym and self.scale_fmt == "fp16" and bits <= 8
                 and group <= 1024 and (group * bits) % 8 == 0 and (width * bits) % 8 == 0 and rows > 0):
