@@ -377,10 +377,21 @@ def dequantize_rows(packed: Tensor, scales: Tensor, values: Tensor, zeros: Tenso
     return out
 
 
+def mix_supported(x: Tensor, signs: Tensor | None, out: Tensor, rows: int, factor: int, power: int) -> bool:
+    """Whether ``mkb_hadamard_mix`` covers a transform whose basis is a Hadamard matrix (the C entry point checks the
+    same), and is the faster kernel for it: a row per CTA needs rows to fill the GPU with.  14336 = 28 x 512 takes 6.1 us
+    with the factor kernel and 7.2 with this one at 16 rows, 9.5 and 7.4 at 32; 18432 = 36 x 512, one CTA per SM, 9.9
+    and 11.1 at 32, 13.0 and 11.3 at 64."""
+    return (rows >= (32 if factor <= 32 else 64) and x.dtype in (torch.float16, torch.bfloat16) and 2 <= factor <= 48
+            and power in (128, 256, 512, 1024) and x.data_ptr() % 16 == 0 and out.data_ptr() % 8 == 0
+            and (signs is None or signs.data_ptr() % 4 == 0))
+
+
 def structured_transform(x: Tensor, *, factor: int, power: int, basis: Tensor | None = None,
                          signs: Tensor | None = None, inverse: bool = False, normalize: bool = True,
-                         out: Tensor | None = None) -> Tensor:
-    """``(basis kron H_power)(x * signs)`` over the last axis, one fused launch; dtype preserved."""
+                         out: Tensor | None = None, hadamard_basis: bool = False) -> Tensor:
+    """``(basis kron H_power)(x * signs)`` over the last axis, one fused launch; dtype preserved.  ``hadamard_basis``
+    says that the entries of ``basis`` are all of one magnitude."""
     device = _require_cuda(x, basis, signs, out)
     width = x.shape[-1]
     if factor * power != width:
@@ -393,8 +404,12 @@ def structured_transform(x: Tensor, *, factor: int, power: int, basis: Tensor | 
     if basis is not None and (basis.dtype != torch.float32 or not basis.is_contiguous()):
         raise ValueError("basis must be a contiguous fp32 matrix")
     rows = source.numel() // width if width else 0
+    library = _native.library()
+    entry = library.mkb_hadamard
+    if hadamard_basis and basis is not None and mix_supported(source, signs, out, rows, factor, power):
+        entry = library.mkb_hadamard_mix
     with torch.cuda.device(device):
-        status = _native.library().mkb_hadamard(
+        status = entry(
             source.data_ptr(), _pointer(signs), _pointer(basis), out.data_ptr(), rows, width, factor,
             power, _tag(x.dtype, "activation"), int(inverse), int(normalize), _stream(device))
     _native.check(status, "structured_transform")

@@ -81,6 +81,13 @@ def transform_factor(width: int) -> tuple[int, int, Tensor | None]:
     return odd, power, matrix.float()
 
 
+@functools.lru_cache(maxsize=128)
+def _hadamard_basis(width: int) -> bool:
+    """Whether the factor basis is a Hadamard matrix up to its scale (a Paley basis, not the DCT)."""
+    basis = transform_factor(width)[2]
+    return basis is not None and bool((basis.abs() == basis.abs()[0, 0]).all())
+
+
 @functools.lru_cache(maxsize=64)
 def _device_basis(width: int, device: torch.device) -> Tensor | None:
     basis = transform_factor(width)[2]
@@ -119,7 +126,7 @@ def structured_transform(value: Tensor, *, inverse: bool = False, signs: Tensor 
     width = value.shape[-1]
     factor, power, _ = transform_factor(width)
     return kernels.structured_transform(value, factor=factor, power=power, basis=_device_basis(width, value.device),
-                                        signs=signs, inverse=inverse)
+                                        signs=signs, inverse=inverse, hadamard_basis=_hadamard_basis(width))
 
 
 def randomized_transform(value: Tensor, *, seed: int = 0, inverse: bool = False,
