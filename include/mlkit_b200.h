@@ -172,7 +172,7 @@ int mkb_gemv_hadamard(const void* x, const int8_t* signs, const uint8_t* packed,
  * in global memory and hands it to a library GEMM (PackedLinear.forward,
  * src/mlkit/inference/packed_linear.py:153-154 with the `weight` property at :110-130).  The weights
  * are rounded to fp16 exactly as that reconstruction rounds them, products are accumulated in fp32
- * on the tensor cores (tcgen05.mma, weights through tensor memory), the result is rounded once.
+ * on the tensor cores (tcgen05.mma), the result is rounded once.
  * Covers symmetric INT4 on the integer grid -8..7 (bits = 4, lut_len = 16, integer_grid = 1,
  * grid_minimum = -8, zeros = null), fp16 activations and scales, group = 128, K a multiple of 128,
  * x and packed 16-byte aligned; anything else returns MKB_E_UNSUPPORTED and the caller keeps the
@@ -192,6 +192,20 @@ int mkb_gemm(const void* x, const uint8_t* packed, const void* scales, const flo
              int integer_grid, float grid_minimum,
              void* workspace, int64_t workspace_bytes, void* stream);
 int mkb_gemm_status(const void* workspace, int* status);
+
+/* The same product for any number of rows and any codec of 2 to 8 bits, offsets included, with fp16 scales per 128, 64 or
+ * 32 codes and fp16 or bf16 activations: weights are rounded to the activations' type as the reconstruction rounds them.
+ * K a multiple of 128, x and packed and its rows 16-byte aligned; anything else returns MKB_E_UNSUPPORTED.
+ * partials: mkb_gemm_tile_partial_bytes(M) bytes of scratch, 16-byte aligned, contents irrelevant.
+ * status: one int on the device, set non-zero when a bounded wait expired (the results are then not valid). */
+int64_t mkb_gemm_tile_partial_bytes(int M);
+int mkb_gemm_tile(const void* x, const uint8_t* packed, const void* scales, const float* lut,
+                  const void* zeros, const void* bias, void* y,
+                  int M, int N, int K, int group, int bits, int lut_len,
+                  int x_dtype, int scale_dtype,
+                  int64_t packed_row_stride, int64_t scale_row_stride,
+                  int integer_grid, float grid_minimum,
+                  void* partials, int64_t partial_bytes, int* status, void* stream);
 
 /*
  * Unpack and dequantise a packed weight:

@@ -24,6 +24,8 @@ SIGNATURES = {
     "mkb_gemv_hadamard": (c_int, [c_void_p] * 7 + [c_int] * 8 + [c_int64, c_int64, c_int, c_float, c_int, c_void_p]),
     "mkb_gemm_workspace_bytes": (c_int64, [c_int] * 3),
     "mkb_gemm": (c_int, [c_void_p] * 7 + [c_int] * 8 + [c_int64, c_int64, c_int, c_float, c_void_p, c_int64, c_void_p]),
+    "mkb_gemm_tile_partial_bytes": (c_int64, [c_int]),
+    "mkb_gemm_tile": (c_int, [c_void_p] * 7 + [c_int] * 8 + [c_int64, c_int64, c_int, c_float, c_void_p, c_int64, c_void_p, c_void_p]),
     "mkb_gemm_status": (c_int, [c_void_p, c_void_p]),
     "mkb_gemv_ws": (c_int, [c_void_p] * 7 + [c_int] * 8 + [c_int64, c_int64, c_int, c_float, c_int, c_void_p, c_int64,
                             c_void_p]),

@@ -21,6 +21,7 @@ from typing import Any
 import torch
 import torch.nn.functional as functional
 from torch import Tensor, nn
+from torch.autograd import forward_ad
 
 from mlkit_b200 import kernels
 from mlkit_b200.models import Model, QModel
@@ -102,6 +103,14 @@ def _packed_matvec_op(x: Tensor, packed: Tensor, scales: Tensor, values: Tensor,
 @_packed_matvec_op.register_fake
 def _(x, packed, scales, values, zeros, bias, outputs, group, bits, integer_grid, grid_minimum):
     return x.new_empty((x.shape[0], outputs))
+
+
+def _plain(inputs: Tensor) -> bool:
+    """Whether nothing but the values of ``inputs`` matters to an operation on it now."""
+    return (type(inputs) in (Tensor, nn.Parameter) and not torch._C._functorch.is_functorch_wrapped_tensor(inputs)
+            and torch._C._len_torch_dispatch_stack() == 0 and not torch.jit.is_tracing()
+            and (forward_ad._current_level < 0 or forward_ad.unpack_dual(inputs).tangent is None)
+            and not (torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") != inputs.dtype))
 
 
 class PackedLinear(nn.Module):
@@ -234,31 +243,29 @@ class PackedLinear(nn.Module):
             raise ValueError("packed inference requires CUDA inputs")
         rows = inputs.numel() // width
         if rows > self.maximum_fused_rows or rows == 0:
-            fused_gemm = (rows > 0 and self.layout is not None and inputs.is_cuda
-                          and kernels.gemm_supported(rows, width=width, group=self.group, bits=self.code_bits,
-                                                     dtype=inputs.dtype, scales=self.scales, zeros=self.zeros,
-                                                     integer_grid=self.integer_grid, grid_minimum=self.grid_minimum,
-                                                     levels=self.values.numel(), outputs=self.out_features))
-            chunked_rows = 2 * self.maximum_fused_rows if fused_gemm else 4 * self.maximum_fused_rows
-            if (0 < rows <= chunked_rows and self.layout is not None and not torch.compiler.is_compiling()
-                    and self._dense_weight is None and not (inputs.requires_grad and torch.is_grad_enabled())
-                    and inputs.dtype == torch.float16 and inputs.is_cuda):
+            eager = (rows > 0 and self.layout is not None and not torch.compiler.is_compiling() and self._dense_weight is None
+                     and not (inputs.requires_grad and torch.is_grad_enabled()))
+            tiled = eager and self._takes_tile_gemm(inputs, rows)
+            chunked_rows = 2 * self.maximum_fused_rows if tiled else 4 * self.maximum_fused_rows
+            if eager and rows <= chunked_rows and inputs.dtype == torch.float16:
                 # a few rows more than one matvec takes: the matvec on chunks of eight rows streams the packed
-                # weight once per chunk, which measured faster than the fused GEMM up to 16 rows (16.9 against
-                # 19.4 us on 4096 -> 14336) and than reconstruct + library GEMM up to 32 rows for every codec
+                # weight once per chunk, which measured faster than the tile GEMM up to 16 rows (16.5 against
+                # 19.5 us on 4096 -> 14336) and than reconstruct + library GEMM up to 32 rows for every codec
                 flat = inputs.reshape(rows, width).contiguous()
                 out = inputs.new_empty((rows, self.out_features))
                 plan = self._plan(inputs.dtype)
                 for start in range(0, rows, self.maximum_fused_rows):
                     plan(flat[start:start + self.maximum_fused_rows], out[start:start + self.maximum_fused_rows])
                 return out.view(inputs.shape[:-1] + (self.out_features,))
-            if (fused_gemm and not torch.compiler.is_compiling() and self._dense_weight is None
-                    and not (inputs.requires_grad and torch.is_grad_enabled())):
-                # up to 128 rows: the weight is reconstructed inside the GEMM kernel, tile by tile
+            if tiled:
+                # the weight is reconstructed inside the GEMM kernel, tile by tile
                 flat = inputs.reshape(rows, width).contiguous()
-                out = kernels.packed_gemm(flat, self.packed, self.scales, self.values, self.bias,
-                                          inputs.new_empty((rows, self.out_features)), group=self.group,
-                                          bits=self.code_bits, integer_grid=True, grid_minimum=self.grid_minimum)
+                if flat.data_ptr() % 16:
+                    flat = flat.clone()
+                out = kernels.packed_tile_gemm(flat, self.packed, self.scales, self.values, self.zeros, self.bias,
+                                               inputs.new_empty((rows, self.out_features)), group=self.group,
+                                               bits=self.code_bits, integer_grid=self.integer_grid,
+                                               grid_minimum=self.grid_minimum)
                 return out.view(inputs.shape[:-1] + (self.out_features,))
             return functional.linear(inputs, self.weight.to(inputs.dtype), self.bias)
         if inputs.requires_grad and torch.is_grad_enabled():
@@ -282,6 +289,27 @@ class PackedLinear(nn.Module):
             else:
                 out = self._plan(inputs.dtype)(flat, inputs.new_empty((rows, self.out_features)))
         return out.view(inputs.shape[:-1] + (self.out_features,))
+
+    def _takes_tile_gemm(self, inputs: Tensor, rows: int) -> bool:
+        dtype = inputs.dtype
+        if (self.packed.data_ptr() % 16 or self.in_features * self.code_bits // 8 % 16
+                or not kernels.tile_gemm_supported(rows, width=self.in_features, group=self.group, bits=self.code_bits,
+                                                   dtype=dtype, scales=self.scales, outputs=self.out_features)):
+            return False
+        form = dict(width=self.in_features, group=self.group, bits=self.code_bits, dtype=dtype, scales=self.scales,
+                    zeros=self.zeros, integer_grid=self.integer_grid, grid_minimum=self.grid_minimum,
+                    levels=self.values.numel())
+        if kernels.gemm_supported(rows, outputs=self.out_features, **form):
+            return True
+        # calls that would reconstruct and use functional.linear: what that sees and this launch does not stays there
+        # (tracers, functional transforms, tangents, autocast, a bias of another type), and a layer that keeps its
+        # reconstruction lets a call make it
+        if self.cache_dense or not _plain(inputs) or not (self.bias is None or self.bias.dtype == dtype):
+            return False
+        # small layers of a codec other than symmetric INT4 g128 in fp16: four matvec launches are as quick, and keep
+        # every row what the matvec gives for it alone
+        return (rows > 4 * self.maximum_fused_rows or dtype != torch.float16 or self.out_features * self.in_features >= 1 << 21
+                or kernels.gemm_supported(rows, **form))
 
     def extra_repr(self) -> str:
         return (f"in_features={self.in_features}, out_features={self.out_features}, bits={self.code_bits}, "

@@ -190,6 +190,53 @@ def packed_gemm(x: Tensor, packed: Tensor, scales: Tensor, values: Tensor, bias:
     return out
 
 
+def _status_word(device: torch.device) -> Tensor:
+    """The head whose last word is the status the tile GEMMs of a (device, stream) share."""
+    key = (device.index if device.index is not None else torch.cuda.current_device(),
+           torch.cuda.current_stream(device).cuda_stream)
+    held = _gemm_workspaces.get(key)
+    if held is None:
+        held = _gemm_workspaces[key] = torch.zeros(1 << 20, dtype=torch.uint8, device=device)
+    return held
+
+
+def tile_gemm_supported(rows: int, *, width: int, group: int, bits: int, dtype: torch.dtype, scales: Tensor,
+                        outputs: int) -> bool:
+    """Whether ``packed_tile_gemm`` covers a layer (the C entry point checks the same and more) and is the faster route.
+    Up to 128 rows it is ahead of reconstruct + library GEMM at every size measured (896 x 896 to 28672 x 4096).
+    Above, both multiply at the tensor cores' rate and what it saves is the reconstruction, so the weight has to be
+    large and the rows few: 4096 x 4096 at 1024 rows 42 us against 44, at 1537 rows 54 against 53; 1024 x 4096 at 512
+    rows 14.3 against 14.5, at 1024 rows 18 against 17."""
+    if not (2 <= bits <= 8 and group in (32, 64, 128) and width % 128 == 0 and dtype in (torch.float16, torch.bfloat16)
+            and scales.dtype == torch.float16):
+        return False
+    return rows <= 128 or (outputs * width >= 1 << 22 and rows <= 512) or (outputs * width >= 1 << 24 and rows <= 1024)
+
+
+def packed_tile_gemm(x: Tensor, packed: Tensor, scales: Tensor, values: Tensor, zeros: Tensor | None, bias: Tensor | None,
+                     out: Tensor, *, group: int, bits: int, integer_grid: bool, grid_minimum: float) -> Tensor:
+    """``out[M, N] = x[M, K] @ dequant(packed)^T (+ bias)`` for any number of rows (``mkb_gemm_tile``); the weight is
+    rounded to the type of ``x`` and never written to memory."""
+    device = _require_cuda(x, packed, scales, values, zeros, bias, out)
+    rows, width = x.shape
+    if not x.is_contiguous() or not out.is_contiguous() or out.dtype != x.dtype or out.shape[0] != rows:
+        raise ValueError("packed_tile_gemm needs contiguous activations and outputs of one type and number of rows")
+    if zeros is not None and zeros.dtype != scales.dtype:
+        raise ValueError("offsets must share the dtype of the scales")
+    if bias is not None and bias.dtype != x.dtype:
+        bias = bias.to(x.dtype)
+    library = _native.library()
+    with torch.cuda.device(device):
+        partials = torch.empty(library.mkb_gemm_tile_partial_bytes(rows), dtype=torch.uint8, device=device)
+        status = library.mkb_gemm_tile(
+            x.data_ptr(), packed.data_ptr(), scales.data_ptr(), values.data_ptr(), _pointer(zeros), _pointer(bias), out.data_ptr(),
+            rows, out.shape[1], width, group, bits, values.numel(), _tag(x.dtype, "activation"), _tag(scales.dtype, "scale"),
+            width * bits // 8, scales.stride(0) if scales.dim() == 2 else -(-width // group), int(integer_grid),
+            float(grid_minimum), partials.data_ptr(), partials.numel(), _status_word(device).data_ptr() + 65532, _stream(device))
+    _native.check(status, "packed_tile_gemm")
+    return out
+
+
 def packed_matvec(x: Tensor, packed: Tensor, scales: Tensor, values: Tensor, zeros: Tensor | None,
                   bias: Tensor | None, out: Tensor, *, group: int, bits: int, integer_grid: bool = False,
                   grid_minimum: float = 0.0, kernel: str = "auto", packed_row_stride: int | None = None,
