@@ -218,6 +218,8 @@ extern "C" int mkb_gemv_hadamard(const void* x, const int8_t* signs, const uint8
   using namespace mkb;
   MKB_REQUIRE(M >= 1 && N >= 1 && K >= 1 && group >= 1, MKB_E_ARGUMENT, "gemv_hadamard: bad shape");
   MKB_REQUIRE(x && packed && scales && lut && y, MKB_E_ARGUMENT, "gemv_hadamard: null pointer");
+  // the plain matvec takes bf16 rows too; the rotating instances exist for fp16 alone
+  MKB_REQUIRE(x_dtype == MKB_F16, MKB_E_UNSUPPORTED, "gemv_hadamard: needs fp16 activations");
   MKB_REQUIRE(gemv_stream_supported(M, N, K, group, bits, lut_len, x_dtype, scale_dtype, x, packed, scales, packed_row_stride,
                                     scale_row_stride, nullptr, integer_grid, grid_minimum) &&
                   gemv_stream_rotation_supported(M, N, K, group, bits, lut_len, integer_grid, grid_minimum, signs),
