@@ -287,8 +287,9 @@ int mkb_hadamard(const void* x, const int8_t* signs, const float* basis, void* y
                  void* stream);
 
 /* The same transform for many 16-bit rows when `basis` is a Hadamard matrix up to its scale (every entry +-b, as a Paley
- * basis has): the F-point mix runs on the tensor cores and a row is read once.  factor 2..48, pow2 128..1024, dtype
- * MKB_F16 or MKB_BF16, x / y / signs on 16 / 8 / 4 byte boundaries; everything else is MKB_E_UNSUPPORTED. */
+ * basis has): the F-point mix runs on the tensor cores and a row is read once.  factor 2..48 with pow2 128, 256 or 512,
+ * factor 2..32 with pow2 1024 (shared memory), dtype MKB_F16 or MKB_BF16, x / y / signs on 16 / 8 / 4 byte boundaries;
+ * everything else is MKB_E_UNSUPPORTED. */
 int mkb_hadamard_mix(const void* x, const int8_t* signs, const float* basis, void* y, int64_t M, int W, int factor,
                      int pow2, int dtype, int inverse, int normalize, void* stream);
 

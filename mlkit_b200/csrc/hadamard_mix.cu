@@ -1,5 +1,6 @@
 // The structured transform  y = (B kron H_P)(x * signs)  of many 16-bit rows whose factor basis is a Hadamard matrix,
-// all entries +-b (a Paley basis): width = F * P with F <= 48, 128 <= P <= 1024.
+// all entries +-b (a Paley basis): width = F * P with F <= 48, 128 <= P <= 1024, and F <= 32 at P = 1024 (the row and
+// its fp32 values have to fit shared memory: 33 x 1024 would need 235 KB of the 227).
 //
 // The factor kernel of hadamard.cu gives a row to ceil(F / 4) CTAs, each of which reads the whole row and spends F
 // multiply-adds per value: at 4096 rows of 14336 = 28 x 512 it is bound by those and by its two-byte loads (450 us).
@@ -243,7 +244,9 @@ int launch_factor(const MixArgs& a, int dtype, cudaStream_t stream) {
     case 128: return launch_mix<FT, 2>(a, dtype, stream);
     case 256: return launch_mix<FT, 4>(a, dtype, stream);
     case 512: return launch_mix<FT, 8>(a, dtype, stream);
-    default: return launch_mix<FT, 16>(a, dtype, stream);
+    default:
+      if constexpr (FT <= 2) return launch_mix<FT, 16>(a, dtype, stream);
+      else MKB_REQUIRE(false, MKB_E_UNSUPPORTED, "hadamard_mix: factors above 32 with 1024 do not fit shared memory");
   }
 }
 

@@ -429,7 +429,8 @@ def mix_supported(x: Tensor, signs: Tensor | None, out: Tensor, rows: int, facto
     same), and is the faster kernel for it: a row per CTA needs rows to fill the GPU with.  14336 = 28 x 512 takes 6.1 us
     with the factor kernel and 7.2 with this one at 16 rows, 9.5 and 7.4 at 32; 18432 = 36 x 512, one CTA per SM, 9.9
     and 11.1 at 32, 13.0 and 11.3 at 64."""
-    return (rows >= (32 if factor <= 32 else 64) and x.dtype in (torch.float16, torch.bfloat16) and 2 <= factor <= 48
+    return (rows >= (32 if factor <= 32 else 64) and x.dtype in (torch.float16, torch.bfloat16)
+            and 2 <= factor <= (32 if power == 1024 else 48)      # shared memory holds a row and its fp32 values
             and power in (128, 256, 512, 1024) and x.data_ptr() % 16 == 0 and out.data_ptr() % 8 == 0
             and (signs is None or signs.data_ptr() % 4 == 0))
 

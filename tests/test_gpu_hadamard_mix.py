@@ -28,6 +28,22 @@ def plain(x, signs, factor, power, basis, inverse):
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("width", [36 * 1024, 44 * 1024])
+def test_widths_that_stay_with_the_factor_kernel(width):
+    """Rows too wide for the shared memory of the tensor-core form, through the public call."""
+    import mlkit_b200 as mk
+    from mlkit_b200 import transforms
+
+    factor, power, basis = transforms.transform_factor(width)
+    assert (factor, power) == (width // 1024, 1024) and transforms._hadamard_basis(width)
+    x, signs = torch.randn(96, width, device="cuda"), (torch.randint(0, 2, (width,), device="cuda") * 2 - 1).to(torch.int8)
+    for dtype in BOUND:
+        for inverse in (False, True):
+            expected = plain(x.to(dtype), signs, factor, power, basis, inverse)
+            got = mk.rht(x.to(dtype), signs=signs, inverse=inverse)
+            assert float((got.double() - expected).norm() / expected.norm()) <= BOUND[dtype]
+
+
 @pytest.mark.parametrize("width", [12 * 128, 44 * 128, 20 * 256, 36 * 256, 28 * 512, 36 * 512, 12 * 1024, 28 * 1024])
 def test_against_64_bits(width, dtype):
     from mlkit_b200 import transforms

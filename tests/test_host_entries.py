@@ -1,8 +1,12 @@
-"""What the C entry points accept and refuse, on the host alone: every check here is made before a launch, so the
-pointers are addresses that nothing reads."""
+"""What the C entry points accept and refuse, on the host alone.  The pointers are addresses that nothing may read, so
+these tests do not run where a device would: there the calls that are accepted would launch."""
 
-from mlkit_b200 import _native
+import pytest
+import torch
 
+from mlkit_b200 import _native, kernels
+
+pytestmark = pytest.mark.skipif(torch.cuda.is_available(), reason="an accepted call would launch on made-up addresses")
 F16, BF16, F32 = _native.F16, _native.BF16, _native.F32
 POINTER, UNSUPPORTED = 1 << 20, -2
 
@@ -18,3 +22,16 @@ def test_rotation_on_load_takes_fp16_rows_only():
         assert rotated(x_dtype) == UNSUPPORTED
         assert b"fp16" in _native.library().mkb_last_error()
     assert rotated(F16, width=14336) == UNSUPPORTED     # and no width with an odd factor
+
+
+def test_many_row_transform_covers_what_its_rule_admits():
+    """The wrapper's rule and the entry point agree at every factor and power (a call that gets as far as the launch
+    fails there: no device)."""
+    x, signs = torch.empty(64, dtype=torch.float16), torch.empty(64, dtype=torch.int8)
+    for power in (64, 128, 256, 512, 1024, 2048):
+        for factor in range(1, 50):
+            for dtype, tag in ((torch.float16, F16), (torch.bfloat16, BF16), (torch.float32, F32)):
+                status = _native.library().mkb_hadamard_mix(POINTER, POINTER, POINTER, POINTER, 64, factor * power, factor,
+                                                            power, tag, 0, 1, None)
+                admitted = kernels.mix_supported(x.to(dtype), signs, x, 64, factor, power)
+                assert (status != UNSUPPORTED) == admitted, (factor, power, dtype)
