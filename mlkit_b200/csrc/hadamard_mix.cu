@@ -16,6 +16,10 @@
 //     while the next row is on its way.
 // Two CTAs share an SM and hide each other's barriers.  4099 rows of 14336 fp16: 451 -> 70 us (3360 GB/s of the
 // 6535 a copy reaches; issue slots bound it), 4099 rows of 6144 = 12 x 512: 128 -> 35 us.
+#include <mutex>
+#include <set>
+#include <utility>
+
 #include "mkb_common.cuh"
 
 namespace mkb {
@@ -212,6 +216,19 @@ __global__ void __launch_bounds__(kMixThreads, mix_residents(FT, NT)) hadamard_m
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
+int opt_in_shared(const void* kernel, int bytes) {
+  static std::mutex lock;
+  static std::set<std::pair<const void*, int>> done;
+  int device = 0;
+  cudaGetDevice(&device);
+  std::lock_guard<std::mutex> guard(lock);
+  if (done.count({kernel, device})) return MKB_OK;
+  const cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (status != cudaSuccess) return cuda_fail(status, "hadamard_mix: shared memory opt-in");
+  done.insert({kernel, device});
+  return MKB_OK;
+}
+
 template <int FT, int NT>
 int launch_mix(const MixArgs& a, int dtype, cudaStream_t stream) {
   auto kernel = dtype == MKB_BF16 ? hadamard_mix_kernel<FT, NT, true> : hadamard_mix_kernel<FT, NT, false>;
@@ -219,9 +236,10 @@ int launch_mix(const MixArgs& a, int dtype, cudaStream_t stream) {
   const size_t smem = size_t(a.F) * PITCH * 4 + size_t(16 * FT) * PITCH * 2;
   const DeviceInfo& info = device_info();
   MKB_REQUIRE(smem <= size_t(info.max_smem_optin), MKB_E_UNSUPPORTED, "hadamard_mix: width %d needs %zu B shared memory", a.W, smem);
-  // (idempotent, and cheap beside the rows this kernel is for)
-  const cudaError_t opted = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-  if (opted != cudaSuccess) return cuda_fail(opted, "hadamard_mix: shared memory opt-in");
+  // once per instance and device and to the device's limit: factors of one instance need different amounts, and a limit
+  // that follows the call could be lowered by another thread before this one launches
+  const int opted = opt_in_shared(reinterpret_cast<const void*>(kernel), info.max_smem_optin);
+  if (opted != MKB_OK) return opted;
   const int64_t resident = int64_t(info.sm_count) * mix_residents(FT, NT);
   cudaLaunchConfig_t config{};
   config.gridDim = dim3(unsigned(a.M < resident ? a.M : resident));

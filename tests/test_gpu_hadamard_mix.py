@@ -92,3 +92,32 @@ def test_not_finite_rows():
     assert torch.equal(got[got.isinf()], general[general.isinf()])
     untouched = [i for i in range(80) if i not in (3, 9, 20)]
     assert torch.equal(got[untouched], clean[untouched])
+
+
+def test_threads_with_factors_of_one_instance():
+    """10240 = 20 x 512 and 14336 = 28 x 512 share a kernel instance and need different amounts of shared memory."""
+    import threading
+
+    from mlkit_b200 import transforms
+
+    inputs = [torch.randn(64, width, device="cuda").half() for width in (10240, 14336)]
+    expected = [transforms.structured_transform(x) for x in inputs]
+    failures = []
+
+    def work(index):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(1500):
+                    got = transforms.structured_transform(inputs[index])
+                torch.cuda.current_stream().synchronize()
+            assert torch.equal(got, expected[index])
+        except Exception as error:
+            failures.append(error)
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(index,)) for index in (0, 1, 0, 1)]
+    for thread in threads:
+        thread.start()
+    for thread in threads:
+        thread.join()
+    assert not failures, failures[0]
