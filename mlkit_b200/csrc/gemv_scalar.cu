@@ -42,11 +42,11 @@ __global__ void __launch_bounds__(kWarps * 32) gemv_scalar_kernel(ScalarArgs a) 
   r.zeros = a.zeros == nullptr ? nullptr
                                : static_cast<const uint8_t*>(a.zeros) + int64_t(row) * a.scale_row_stride * dtype_bytes(a.scale_dtype);
   r.lut = lut_s; r.lut_len = 256;
-  r.K = a.K; r.group = a.group; r.bits = a.bits; r.x_dtype = a.x_dtype; r.scale_dtype = a.scale_dtype;
+  r.K = a.K; r.group = a.group; r.bits = a.bits; r.scale_dtype = a.scale_dtype;
   float acc[MT];
 #pragma unroll
   for (int m = 0; m < MT; ++m) acc[m] = 0.f;
-  scalar_row_products<MT>(r, a.x, a.M, lane, acc);
+  scalar_row_products<MT>(r, [&](int m, int k) { return load_as_float(a.x, int64_t(m) * a.K + k, a.x_dtype); }, a.M, lane, acc);
 #pragma unroll
   for (int m = 0; m < MT; ++m)
     for (int offset = 16; offset; offset >>= 1) acc[m] += __shfl_xor_sync(0xffffffffu, acc[m], offset);

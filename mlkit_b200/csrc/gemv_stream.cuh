@@ -129,9 +129,11 @@ enum { MODE_RAW = 0, MODE_TABLE = 1 };
 //   low, 22 bits), its products are formed per scale group and the fp32 scale multiplies the group's sum:
 //   neither a level nor a scaled weight is rounded to 16 bits.  Cost, 4096 -> 14336 at one row: 8.7 us against 8.0
 //   with fp16 (the max, the move and two shuffles before the first step), 16.7 against 12.3 for NF4 (two parts per
-//   gather); the general kernel, which bf16 took before, needs 140 us.  A row with an infinity or a NaN is redone
-//   after the last visit with plain fp32 products (an infinity times code - minimum is not infinity times code
-//   minus infinity times minimum).
+//   gather); the general kernel, which bf16 took before, needs 140 us.
+// Infinities and NaNs.  An infinity times (code + minimum) is a signed infinity, but the masks form infinity times code
+// plus infinity times minimum, which is a NaN.  With bf16, and with fp16 in the forms of RAW that have several scale
+// groups or offsets, a row with such a value is redone after the last visit with plain fp32 products, whose answer is
+// that of whole weights.  fp16 with one scale per 128 codes and no offset keeps the masks' answer.
 enum { X_F16 = 0, X_BF16 = 1 };
 
 // Geometry of one visit of one warp: 16 rows x KT k-tiles of 128 codes.  GPT = scale groups per k-tile.
@@ -284,6 +286,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) gemv_stream_kernel(const St
   constexpr bool ROTATE = FORM == FORM_ROTATED, GATED = FORM == FORM_GATED;
   constexpr int SPLIT = GROUPED ? GPT : 1;
   constexpr bool RAW = MODE == MODE_RAW;
+  constexpr bool REDO = BF || (RAW && (GPT > 1 || ZERO));   // rows that are not finite are redone
   // dependents may become resident at once: they only copy constants until their own wait returns
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -913,6 +916,22 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) gemv_stream_kernel(const St
     }
   };
 
+  // activation rows that are not finite in this lane's view of this warp's slice, a bit each
+  [[maybe_unused]] auto redo_rows = [&]() -> uint32_t {
+    uint32_t rows = 0;
+    if constexpr (BF) {
+      rows = unbounded ? 1u << g : 0u;
+    } else if constexpr (REDO) {   // the sums of the activations tell
+#pragma unroll
+      for (int kk = 0; kk < KT; ++kk)
+#pragma unroll
+        for (int group = 0; group < V::SUMS; ++group)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) rows |= isfinite(start[kk][group][j]) ? 0u : 1u << (2 * t + j);
+    }
+    return rows;
+  };
+  [[maybe_unused]] int redo = 0;   // whether any warp of the CTA has one
   int batch_first = 0;   // first visit of the batch whose sums shared memory holds
   for (int visit0 = 0; visit0 < a.visits; visit0 += R) {
     const uint32_t red_at = red_to + (visit0 - batch_first) * 512;
@@ -921,7 +940,8 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) gemv_stream_kernel(const St
     if (visit0 + R - batch_first < a.batch && visit0 + R < a.visits) continue;
 
     // ---- end of a batch: add the warps' partial sums in warp order, four outputs per thread ----
-    __syncthreads();
+    if constexpr (REDO) redo = __syncthreads_or(redo_rows() != 0);
+    else __syncthreads();
     const int in_batch = min(a.batch, a.visits - batch_first);
     const int quads = in_batch * a.RG * 32;
     for (int o = threadIdx.x; o < quads; o += blockDim.x) {
@@ -973,12 +993,22 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) gemv_stream_kernel(const St
     cluster.sync();  // no CTA leaves while a peer may still read its sums
   }
 
-  // ---- bf16 rows with an infinity or a NaN: plain products over the whole row, one warp per output.  The CTAs of
-  // a cluster that saw one write the same values, after the barrier above ----
-  if constexpr (BF) {
-    if (__syncthreads_or(unbounded)) {
+  // ---- rows with an infinity or a NaN: plain products over the whole row, one warp per output.  The CTAs of a
+  // cluster that saw one write the same values, after the barrier above ----
+  if constexpr (REDO) {
+    if (redo) {
+      auto activation = [&](int m, int k) -> float {
+        const int64_t at = int64_t(m) * (GATED ? 2 * a.K : a.K) + k;
+        if constexpr (BF) return load_as_float(a.x, at, MKB_BF16);
+        else if constexpr (ROTATE) return __half2float(__float2half_rn(rotated[m * a.K + k]));
+        else if constexpr (GATED) {
+          const uint32_t pair = swiglu_pair(a.x[at], a.x[at + a.K]);
+          return __half2float(__ushort_as_half((unsigned short)(pair & 0xffffu)));
+        } else return load_as_float(a.x, at, MKB_F16);
+      };
+      const uint32_t mine = redo_rows();
       for (int m = 0; m < a.M; ++m) {
-        if (!__syncthreads_or(unbounded && g == m)) continue;
+        if (!__syncthreads_or((mine >> m) & 1u)) continue;
         for (int index = warp; index < a.visits * a.RG * 16; index += warps) {
           const int rt = int(blockIdx.x) * a.RG + (index >> 4) % a.RG + (index >> 4) / a.RG * visit_stride;
           const int row = rt * 16 + (index & 15);
@@ -988,14 +1018,14 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) gemv_stream_kernel(const St
           r.scales = a.scales + int64_t(row) * a.scale_row_stride;
           r.zeros = ZERO ? a.zeros + int64_t(row) * a.scale_row_stride : nullptr;
           r.lut = a.lut; r.lut_len = a.lut_len;
-          r.K = a.K; r.group = a.group; r.bits = a.bits; r.x_dtype = MKB_BF16; r.scale_dtype = MKB_F16;
+          r.K = a.K; r.group = a.group; r.bits = a.bits; r.scale_dtype = MKB_F16;
           float sum[1] = {0.f};
-          scalar_row_products<1>(r, a.x + int64_t(m) * a.K, 1, lane, sum);
+          scalar_row_products<1>(r, [&](int, int k) { return activation(m, k); }, 1, lane, sum);
 #pragma unroll
           for (int offset = 16; offset; offset >>= 1) sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], offset);
           if (lane == 0) {
-            if (a.bias != nullptr) sum[0] += __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(a.bias)[row]);
-            reinterpret_cast<__nv_bfloat16*>(a.y)[int64_t(m) * a.N + row] = __float2bfloat16_rn(sum[0]);
+            if (a.bias != nullptr) sum[0] += load_as_float(a.bias, row, BF ? MKB_BF16 : MKB_F16);
+            store_from_float(a.y, int64_t(m) * a.N + row, BF ? MKB_BF16 : MKB_F16, sum[0]);
           }
         }
       }

@@ -11,13 +11,14 @@ struct ScalarRow {   // one weight row
   const void* scales;
   const void* zeros;      // offsets or null
   const float* lut;       // `lut_len` levels; a code past the end stands for zero
-  int K, group, bits, lut_len, x_dtype, scale_dtype;
+  int K, group, bits, lut_len, scale_dtype;
 };
 
 // Adds the products of the words lane, lane + 32, ... to acc[0..M): w = lut[c] * scale (+ zero), one fp32 rounding
-// each, then a fused multiply-add per activation row.  x: M rows of K.
-template <int MT>
-__device__ __forceinline__ void scalar_row_products(const ScalarRow& r, const void* x, int M, int lane, float (&acc)[MT]) {
+// each, then a fused multiply-add per activation row.  activation(m, k) is element k of activation row m.
+template <int MT, typename Activation>
+__device__ __forceinline__ void scalar_row_products(const ScalarRow& r, const Activation& activation, int M, int lane,
+                                                    float (&acc)[MT]) {
   const int wb = word_bytes(r.bits), wc = word_codes(r.bits);
   const int words = r.K / wc;
   const uint32_t mask = (1u << r.bits) - 1u;
@@ -35,7 +36,7 @@ __device__ __forceinline__ void scalar_row_products(const ScalarRow& r, const vo
       const float weight = has_zero ? reconstruct(value, scale, zero) : reconstruct(value, scale);
 #pragma unroll
       for (int m = 0; m < MT; ++m)
-        if (m < M) acc[m] = fmaf(weight, load_as_float(x, int64_t(m) * r.K + k0 + c, r.x_dtype), acc[m]);
+        if (m < M) acc[m] = fmaf(weight, activation(m, k0 + c), acc[m]);
     }
   }
 }

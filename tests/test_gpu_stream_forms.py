@@ -107,6 +107,61 @@ def test_bf16_infinities_and_nans(kind, bits, group, zeros, width):
     assert got[0].isinf().any()
 
 
+@pytest.mark.parametrize("width", [128, 1024, 9216])
+@pytest.mark.parametrize("kind,bits,group,zeros", [("int", 4, 64, False), ("int", 4, 32, False), ("int", 4, 128, True),
+                                                   ("int", 4, 64, True), ("int", 4, 32, True), ("nf4", 4, 64, False)])
+def test_fp16_infinities_and_nans(kind, bits, group, zeros, width):
+    """The same with fp16, in the forms that once took kernels of whole weights: an infinity stays a signed infinity."""
+    generator = torch.Generator(device="cuda").manual_seed(6)
+    layer = layer_of(kind, bits, group, zeros, 100, width)
+    x = torch.randn(8, width, generator=generator, device="cuda").half()
+    clean = run(layer, x)
+    dirty = x.clone()
+    dirty[0, 77] = float("inf")
+    dirty[1, width - 1], dirty[1, 5] = float("-inf"), float("nan")
+    dirty[3, 20], dirty[3, 30] = float("inf"), float("-inf")
+    dirty[7, 0] = float("-inf")
+    got, general = run(layer, dirty), run(layer, dirty, kernel="scalar")
+    assert torch.equal(got[[2, 4, 5, 6]], clean[[2, 4, 5, 6]])
+    for row in (0, 1, 3, 7):
+        assert torch.equal(got[row].isnan(), general[row].isnan())
+        finite = ~general[row].isnan()
+        assert torch.equal(got[row][finite], general[row][finite])
+    assert got[0].isinf().any() and got[7].isinf().any() and not got[7, layer["dense"][:, 0] != 0].isnan().any()
+
+
+@pytest.mark.parametrize("kind,group", [("int", 64), ("nf4", 64)])
+def test_gated_and_rotated_rows_that_are_not_finite(kind, group):
+    """Forms that make their activations on load: the gate's product overflows to an infinity, or an input is one."""
+    from mlkit_b200 import kernels
+
+    generator = torch.Generator(device="cuda").manual_seed(8)
+    layer = layer_of(kind, 4, group, False, 100, 1024)
+    integer, low = kernels.integer_grid_of(layer["values"])
+    form = dict(group=group, bits=4, integer_grid=integer, grid_minimum=low)
+    held = layer["packed"], layer["scales"], layer["values"], None
+
+    def gated(both):
+        out = torch.full((both.shape[0], 100), float("nan"), dtype=torch.float16, device="cuda")
+        return kernels.packed_matvec(both, *held, None, out, gated=True, **form)
+
+    both = torch.randn(3, 2048, generator=generator, device="cuda").half()
+    clean = gated(both)
+    both[1, 7], both[1, 1024 + 7] = 600.0, -600.0          # fp16 ends at 65504
+    got, weights = gated(both), layer["dense"][:, 7]
+    assert torch.equal(got[[0, 2]], clean[[0, 2]])
+    assert torch.equal(got[1].isnan(), weights == 0)
+    assert torch.equal(got[1][weights != 0].double(), weights[weights != 0].sign() * float("-inf"))
+
+    x = torch.randn(3, 1024, generator=generator, device="cuda").half()
+    x[1, 9] = float("inf")
+    signs = (torch.randint(0, 2, (1024,), generator=generator, device="cuda") * 2 - 1).to(torch.int8)
+    out = torch.empty(3, 100, dtype=torch.float16, device="cuda")
+    kernels.packed_matvec_rotated(x, signs, *held, out, **form)
+    expected = run(layer, kernels.structured_transform(x, factor=1, power=1024, signs=signs))
+    assert torch.equal(out.isnan(), expected.isnan()) and torch.equal(out.nan_to_num(), expected.nan_to_num())
+
+
 def test_forms_left_to_other_kernels():
     """Layouts outside the streaming kernel still answer, and its explicit choice refuses what it refused."""
     generator = torch.Generator(device="cuda").manual_seed(7)
