@@ -1,6 +1,9 @@
 """What the C entry points accept and refuse, on the host alone.  The pointers are addresses that nothing may read, so
 these tests do not run where a device would: there the calls that are accepted would launch."""
 
+import re
+from pathlib import Path
+
 import pytest
 import torch
 
@@ -35,3 +38,14 @@ def test_many_row_transform_covers_what_its_rule_admits():
                                                             power, tag, 0, 1, None)
                 admitted = kernels.mix_supported(x.to(dtype), signs, x, 64, factor, power)
                 assert (status != UNSUPPORTED) == admitted, (factor, power, dtype)
+
+
+def test_bounded_waits_of_the_tile_gemm_end_for_whole_warps():
+    """By reading the source, an expired wait being nothing to bring about on a device: wherever the outcome of a wait
+    decides what its lanes do next it is voted on by the warp, and what is left of the plain wait only waits."""
+    source = (Path(kernels.__file__).parent / "csrc" / "gemm_tile.cu").read_text()
+    uses = [line.strip() for line in source.splitlines() if re.search(r"\btile_wait\(", line)]
+    deciding = [line for line in uses if not line.startswith("tile_wait(")]
+    assert deciding == ["__device__ __forceinline__ bool tile_wait(uint64_t* bar, uint32_t parity, volatile int* failed) {",
+                        "return __all_sync(0xffffffffu, tile_wait(bar, parity, failed));"]
+    assert "__all_sync(0xffffffffu, tile_wait" in source and source.count("tile_wait_warp(") > 5
