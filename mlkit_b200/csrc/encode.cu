@@ -16,6 +16,8 @@
 //    flag for infinities and NaNs are formed on the way.
 //  * group kernel (every other group): one warp per group, a pass for the range, a pass for the codes (through
 //    shared memory), then each lane assembles whole bytes of the stream.
+#include <cfloat>
+
 #include "mkb_common.cuh"
 
 namespace mkb {
@@ -178,9 +180,9 @@ __global__ void __launch_bounds__(kRunThreads) rtn_encode_runs_kernel(const Enco
 #pragma unroll
   for (int j = 0; j < kRunsPerThread; ++j) {
     bad |= largest[j] >= 0x7f800000u;
-    float low = INFINITY, range;
+    [[maybe_unused]] float low = INFINITY, high = -INFINITY;
+    float range;
     if constexpr (ASYM) {
-      float high = -INFINITY;
       if (live[j]) {
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
@@ -217,10 +219,22 @@ __global__ void __launch_bounds__(kRunThreads) rtn_encode_runs_kernel(const Enco
     // codes as the low bits of `code` once `base` is taken away (of all of them at once, modulo the word)
     uint32_t code[8];
     constexpr uint32_t base = INTEGER ? kRoundMagicBits : 0u;
-    const float inverse = __frcp_rn(scale);
+    float divisor = scale, moved = offset;
+    if constexpr (ASYM) {
+      // a narrow group far from zero: its offset ends at fp16's largest value and quotients by a scale of 2^-24 can
+      // overflow, which the correction would turn into NaNs.  (Without an offset a scale grows with the weights.)
+      if (fmaxf(fabsf(low), fabsf(high)) >= 1e31f) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          w[j][e] = fminf(fmaxf(__fdiv_rn(__fsub_rn(w[j][e], offset), scale), -FLT_MAX), FLT_MAX);
+        divisor = 1.f;
+        moved = 0.f;
+      }
+    }
+    const float inverse = __frcp_rn(divisor);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      const float q = quotient(ASYM ? __fsub_rn(w[j][e], offset) : w[j][e], scale, inverse);
+      const float q = quotient(ASYM ? __fsub_rn(w[j][e], moved) : w[j][e], divisor, inverse);
       if constexpr (INTEGER) code[e] = __float_as_uint(__fadd_rn(fminf(fmaxf(q, a.low), a.high), kRoundMagic));
       else code[e] = uint32_t(nearest_level(q, level_s, a.level_count));
     }

@@ -60,6 +60,19 @@ def test_quotients_at_rounding_boundaries(bits):
     same(fmt(weight.cuda()), fmt(weight), bits)
 
 
+@pytest.mark.parametrize("kind,bits", [("int", 4), ("int", 8), ("nf4", 4), ("codebook3", 3)])
+def test_narrow_groups_far_from_zero(kind, bits):
+    """Their offset ends at fp16's largest value, the scale at its smallest, and w - offset over it overflows."""
+    weight = torch.full((6, 128), 0.5)
+    weight[0], weight[1], weight[2], weight[3], weight[4, 5] = 1e33, -1e33, 3e38, 2e31, 1e30
+    weight[1, 7] = -1.0009765625e33
+    weight[5, :64] = torch.linspace(-3e38, 3e38, 64) / 2
+    for dtype in (torch.float32, torch.bfloat16):
+        for group in (64, 128):
+            fmt = format_of(kind, bits, group, True)
+            same(fmt(weight.to(dtype).cuda()), fmt(weight.to(dtype)), bits)
+
+
 def test_layouts_and_refusals():
     import mlkit_b200 as mk
 
