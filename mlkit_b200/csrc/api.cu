@@ -145,13 +145,21 @@ extern "C" int mkb_gemv_ws(const void* x, const uint8_t* packed, const void* sca
               "gemv: K=%d or group=%d splits a packing word of %d-bit codes", K, group, bits);
   MKB_REQUIRE(K > 0, MKB_E_UNSUPPORTED, "gemv: empty reduction");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const bool stream_ok = (!gated || (x_dtype == MKB_F16 && zeros == nullptr && group >= 64)) && gemv_stream_supported(M, N, K, group, bits, lut_len, x_dtype, scale_dtype, x, packed, scales,
-                                               packed_row_stride, scale_row_stride, zeros, integer_grid, grid_minimum);
+  const bool stream_ok =
+      (!gated || (x_dtype == MKB_F16 && zeros == nullptr && group >= 64)) &&
+      gemv_stream_supported(M, N, K, group, bits, lut_len, x_dtype, scale_dtype, x, packed, scales, packed_row_stride,
+                            scale_row_stride, zeros, integer_grid, grid_minimum);
   if (kernel == MKB_GEMV_STREAM)   // by name: fp16 activations without offsets and one or two scales per 128 codes
-    MKB_REQUIRE(stream_ok && x_dtype == MKB_F16 && zeros == nullptr && group >= 64, MKB_E_UNSUPPORTED, "gemv: the streaming kernel does not cover these arguments");
-  if (kernel == MKB_GEMV_STREAM || (kernel == MKB_GEMV_AUTO && stream_ok))
-    return launch_gemv_stream(x, packed, scales, lut, zeros, bias, y, M, N, K, group, bits, lut_len, x_dtype,
-                              packed_row_stride, scale_row_stride, integer_grid, grid_minimum, gated, s);
+    MKB_REQUIRE(stream_ok && x_dtype == MKB_F16 && zeros == nullptr && group >= 64, MKB_E_UNSUPPORTED,
+                "gemv: the streaming kernel does not cover these arguments");
+  if (kernel == MKB_GEMV_STREAM || (kernel == MKB_GEMV_AUTO && stream_ok)) {
+    const int launched = launch_gemv_stream(x, packed, scales, lut, zeros, bias, y, M, N, K, group, bits, lut_len, x_dtype,
+                                            packed_row_stride, scale_row_stride, integer_grid, grid_minimum, gated, s);
+    // the launch knows how many clusters the GPU holds and refuses, before it launches anything, a split of K whose
+    // fewer clusters would need too many visits (8 CTAs a cluster: 16 clusters in place of 18, N above 32768): under
+    // AUTO such a call takes a kernel that covers it
+    if (launched != MKB_E_UNSUPPORTED || kernel == MKB_GEMV_STREAM || gated) return launched;
+  }
   const bool tiled_ok = gemv_tiled_supported(M, K, group, bits, x_dtype, scale_dtype, x, packed, packed_row_stride);
   const bool tmem_ok = workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) % 16) == 0 && lut_len == 16 &&
                        gemv_umma_supported(M, K, group, bits, x_dtype, scale_dtype, x, packed, packed_row_stride, zeros,

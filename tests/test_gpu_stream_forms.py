@@ -181,3 +181,21 @@ def test_forms_left_to_other_kernels():
     # a base address off the 16-byte boundary takes the general kernel
     x = torch.randn(2 * 256 + 1, generator=generator, device="cuda").bfloat16()[1:].view(2, 256)
     assert rel(run(layer, x), x.double() @ layer["dense"].t()) <= BOUND[torch.bfloat16]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("outputs", [32768, 34816, 36864])
+def test_wide_layers_of_long_rows(outputs, dtype):
+    """K of 32768 is split over clusters of eight CTAs; how many of those the GPU holds decides whether a launch of this
+    width needs more visits than it keeps sums for, and such a call takes another kernel."""
+    generator = torch.Generator(device="cuda").manual_seed(11)
+    width = 32768
+    packed = torch.randint(0, 256, (outputs * width // 2,), generator=generator, device="cuda", dtype=torch.uint8)
+    scales = (torch.rand(outputs, width // 128, generator=generator, device="cuda") * 0.01 + 0.001).half()
+    layer = {"packed": packed, "scales": scales, "values": torch.arange(-8, 8, device="cuda").float(), "zeros": None,
+             "bits": 4, "group": 128, "outputs": outputs}
+    x = torch.randn(2, width, generator=generator, device="cuda").to(dtype)
+    got = run(layer, x)
+    for first in (0, outputs - 48):
+        part = {**layer, "packed": packed[first * width // 2:(first + 48) * width // 2], "scales": scales[first:first + 48], "outputs": 48}
+        assert rel(got[:, first:first + 48], run(part, x, kernel="scalar").double()) <= 2 * BOUND[dtype]
