@@ -125,9 +125,10 @@ enum { MODE_RAW = 0, MODE_TABLE = 1 };
 //   magnitude of the row's slice into [2^14, 2^15): every value down to 2^-31 of that maximum is then exact
 //   (eight significant bits fit fp16's eleven, its subnormals included), smaller ones err by at most 2^-39 of
 //   it, below what the fp32 accumulation resolves; the warp's sums are moved back before they are added up.
-//   So every decoder of this file serves both types.  A table codec is held as two fp16 parts (level = high +
-//   low, 22 bits), its products are formed per scale group and the fp32 scale multiplies the group's sum:
-//   neither a level nor a scaled weight is rounded to 16 bits.  Cost, 4096 -> 14336 at one row: 8.7 us against 8.0
+//   So every decoder of this file serves both types.  A table codec is held as two fp16 parts, level = high + low to
+//   22 bits, of the table times the power of two that brings its largest level into [2^14, 2^15): a level keeps
+//   the 22 bits down to 2^-27 of the largest, a smaller one errs by at most 2^-39 of it.  Its products are formed per
+//   scale group and the fp32 scale multiplies the group's sum.  Cost, 4096 -> 14336 at one row: 8.7 us against 8.0
 //   with fp16 (the max, the move and two shuffles before the first step), 16.7 against 12.3 for NF4 (two parts per
 //   gather); the general kernel, which bf16 took before, needs 140 us.
 // Infinities and NaNs.  An infinity times (code + minimum) is a signed infinity, but the masks form infinity times code
@@ -362,14 +363,14 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) gemv_stream_kernel(const St
     if (d < a.early) issue(d, d, d < my_visits, d < whole_visits);
 
   // ---- the pair table of the table codecs: entry (lo | hi << BITS) = fp16 (lut[lo], lut[hi]) ----
-  [[maybe_unused]] int table_exponent = 0;   // bf16: the table holds levels * 2^-table_exponent, the largest in [1, 2)
+  [[maybe_unused]] int table_exponent = 0;   // bf16: the table holds levels * 2^-table_exponent, the largest in [2^14, 2^15)
   if constexpr (!RAW) {
     __half2* table = reinterpret_cast<__half2*>(smem + (table_base - smem_base));
     // lane c holds level c: one load instead of two per entry (a warp's entry is the same for all its lanes)
     float level = lane < a.lut_len ? a.lut[lane] : 0.f;
     if constexpr (BF) {
       const uint32_t largest = __reduce_max_sync(0xffffffffu, __float_as_uint(level) & 0x7fffffffu);
-      table_exponent = min(max(int(largest >> 23) - 127, -100), 100);
+      table_exponent = min(max(int(largest >> 23) - 141, -114), 86);
       level *= power_of_two(-table_exponent);
     }
     for (int entry = warp; entry < V::TABLE_ENTRIES; entry += warps) {

@@ -84,6 +84,27 @@ def test_bf16_range(kind, bits, group, zeros):
     assert torch.equal(got[3], torch.zeros_like(got[3]))
 
 
+@pytest.mark.parametrize("bits,group", [(4, 64), (4, 128), (3, 64), (3, 128)])
+def test_bf16_tables_of_far_apart_levels(bits, group):
+    """Levels down to 2^-36 of the largest, in weight rows that hold levels of one size each.  A level is held to 22
+    bits or to 2^-39 of the largest: at 2^-30 that is 2^-9 of it, beside the output's own 2^-8."""
+    from mlkit_b200 import pack
+
+    generator = torch.Generator(device="cuda").manual_seed(9)
+    layer = layer_of("codebook3" if bits == 3 else "nf4", bits, group, False, 64, 1024)
+    sizes = 2.0 ** torch.tensor([0, -10, -20, -24, -25, -27, -30, -36], device="cuda")
+    values = torch.cat((1.3 * sizes, sizes)) if bits == 4 else 1.3 * sizes
+    pairs = torch.randint(0, 2, (64, 1024), generator=generator, device="cuda") * (8 if bits == 4 else 0)
+    codes = (torch.arange(64, device="cuda")[:, None] % 8 + pairs).to(torch.uint8)
+    layer.update(values=values, packed=pack(codes, bits))
+    layer["dense"] = values.double()[codes.long()] * layer["scales"].double().repeat_interleave(group, 1)
+    x = torch.rand(3, 1024, generator=generator, device="cuda").bfloat16()
+    got, expected = run(layer, x), x.double() @ layer["dense"].t()
+    for size in range(7):
+        assert rel(got[:, size::8], expected[:, size::8]) <= BOUND[torch.bfloat16] + 2.0**-9, float(sizes[size])
+    assert rel(got[:, 7::8], expected[:, 7::8]) <= 2.0**-2     # 2^-36 is held to an eighth of itself
+
+
 @pytest.mark.parametrize("width", [1024, 9216])
 @pytest.mark.parametrize("kind,bits,group,zeros", [("int", 4, 128, False), ("int", 4, 64, True), ("int", 3, 128, False),
                                                    ("nf4", 4, 64, False)])
