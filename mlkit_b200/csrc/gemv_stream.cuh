@@ -127,7 +127,7 @@ enum { MODE_RAW = 0, MODE_TABLE = 1 };
 //   it, below what the fp32 accumulation resolves; the warp's sums are moved back before they are added up.
 //   So every decoder of this file serves both types.  A table codec is held as two fp16 parts, level = high + low to
 //   22 bits, of the table times the power of two that brings its largest level into [2^14, 2^15): a level keeps
-//   the 22 bits down to 2^-27 of the largest, a smaller one errs by at most 2^-39 of it.  Its products are formed per
+//   the 22 bits down to 2^-17 of the largest, a smaller one errs by at most 2^-39 of it.  Its products are formed per
 //   scale group and the fp32 scale multiplies the group's sum.  Cost, 4096 -> 14336 at one row: 8.7 us against 8.0
 //   with fp16 (the max, the move and two shuffles before the first step), 16.7 against 12.3 for NF4 (two parts per
 //   gather); the general kernel, which bf16 took before, needs 140 us.
