@@ -443,8 +443,12 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) gemv_stream_kernel(const St
   }
   uint32_t b[KT][16];     // tensor-core step s of a k-tile multiplies by b[2s], b[2s + 1]
   // RAW: sum(x) * 2^-24 of a k-tile's scale group for activation rows 2t, 2t + 1; without offsets already times
-  // the grid minimum, which makes it the accumulators' start
-  float start[KT][V::SUMS][2];
+  // the grid minimum, which makes it the accumulators' start.  With one group it is held twice, as the four registers
+  // in a row that a tensor-core step starts from: put together in the loop they cost the plain matvec 1-2 % (8 rows of
+  // 4096 -> 6144: 5.53 us against 5.40).  3 and 8 bits are short of registers and, like single k-tiles per visit,
+  // quicker with pairs.
+  constexpr int STARTS = V::SUMS == 1 && !ZERO && KT == 2 && BITS != 3 && BITS != 8 ? 4 : 2;
+  float start[KT][V::SUMS][STARTS];
   [[maybe_unused]] float down[2] = {1.f, 1.f};   // bf16: what moves the sums of activation rows 2t, 2t + 1 back
   [[maybe_unused]] bool unbounded = false;       // bf16: row g has an infinity or a NaN in this warp's slice
   // where the eight activations opposite 16-byte piece w of a lane's 64 start in the k-tile
@@ -575,8 +579,8 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) gemv_stream_kernel(const St
 #pragma unroll
           for (int step = STEPS * group + 1; step < STEPS * (group + 1); ++step)
             mma_next(sums, ones, ones, ones, ones, all[2 * step], all[2 * step + 1]);
-          start[kk][group][0] = sums[0] * unit;   // rows g and g + 8 of the tile of ones give the same sums
-          start[kk][group][1] = sums[1] * unit;
+#pragma unroll
+          for (int j = 0; j < STARTS; ++j) start[kk][group][j] = sums[j] * unit;   // rows g and g + 8 have the same sums
         }
       }
     }
@@ -640,7 +644,9 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) gemv_stream_kernel(const St
         }
       };
       // the accumulators' start of a group: min * sum(x), in units of 2^-24
-      auto begin = [&](int group, int row) { return ZERO ? a.grid_min * start[kk][group][row] : start[kk][group][row]; };
+      auto begin = [&](int group, int q) {
+        return ZERO ? a.grid_min * start[kk][group][q & 1] : start[kk][group][q & (STARTS - 1)];
+      };
       if constexpr (BITS == 4) {
         uint32_t q[4], p[4];
 #pragma unroll
@@ -652,9 +658,9 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) gemv_stream_kernel(const St
         for (int w = 0; w < 4; ++w) {
           const uint32_t q8 = q[w] >> 8, p8 = p[w] >> 8;  // codes 2, 3, 6, 7 of a word move down one byte
           if (w % (4 / V::SUMS) == 0) {
-            const float s0 = begin(w * V::SUMS / 4, 0), s1 = begin(w * V::SUMS / 4, 1);
+            const int group = w * V::SUMS / 4;
             mma_first(acc[0], q[w] & 0x000f000fu, p[w] & 0x000f000fu, q8 & 0x000f000fu, p8 & 0x000f000fu,
-                      b[kk][4 * w], b[kk][4 * w + 1], s0, s1, s0, s1);
+                      b[kk][4 * w], b[kk][4 * w + 1], begin(group, 0), begin(group, 1), begin(group, 2), begin(group, 3));
             mma_first(acc[1], q[w] & 0x00f000f0u, p[w] & 0x00f000f0u, q8 & 0x00f000f0u, p8 & 0x00f000f0u,
                       b[kk][4 * w + 2], b[kk][4 * w + 3], 0.f, 0.f, 0.f, 0.f);
           } else {
@@ -675,7 +681,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) gemv_stream_kernel(const St
         for (int step = 0; step < 8; ++step) {
           const uint32_t a0 = __byte_perm(q[step], 0u, 0x4140), a1 = __byte_perm(p[step], 0u, 0x4140);
           const uint32_t a2 = __byte_perm(q[step], 0u, 0x4342), a3 = __byte_perm(p[step], 0u, 0x4342);
-          if (step == 0) mma_first(acc[0], a0, a1, a2, a3, b[kk][0], b[kk][1], begin(0, 0), begin(0, 1), begin(0, 0), begin(0, 1));
+          if (step == 0) mma_first(acc[0], a0, a1, a2, a3, b[kk][0], b[kk][1], begin(0, 0), begin(0, 1), begin(0, 2), begin(0, 3));
           else mma_next(acc[0], a0, a1, a2, a3, b[kk][2 * step], b[kk][2 * step + 1]);
         }
       } else if constexpr (BITS == 3) {
@@ -701,7 +707,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) gemv_stream_kernel(const St
           constexpr uint32_t mask = 0x00070007u << o;
           if constexpr (o == 0)
             mma_first(acc[o], x0 & mask, x1 & mask, y0 & mask, y1 & mask, b[kk][2 * c], b[kk][2 * c + 1],
-                      begin(0, 0), begin(0, 1), begin(0, 0), begin(0, 1));
+                      begin(0, 0), begin(0, 1), begin(0, 2), begin(0, 3));
           else
             mma_first(acc[o], x0 & mask, x1 & mask, y0 & mask, y1 & mask, b[kk][2 * c], b[kk][2 * c + 1], 0.f, 0.f, 0.f, 0.f);
         };
@@ -735,7 +741,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) gemv_stream_kernel(const St
           const uint32_t a2 = (paired_window<BITS, S::window(c1)>(q) >> S::shift(c1)) & mask;
           const uint32_t a3 = (paired_window<BITS, S::window(c1)>(p) >> S::shift(c1)) & mask;
           if constexpr (s == 0)
-            mma_first(acc[o], a0, a1, a2, a3, b[kk][0], b[kk][1], begin(0, 0), begin(0, 1), begin(0, 0), begin(0, 1));
+            mma_first(acc[o], a0, a1, a2, a3, b[kk][0], b[kk][1], begin(0, 0), begin(0, 1), begin(0, 2), begin(0, 3));
           else if constexpr (S::opens_class(s))
             mma_first(acc[o], a0, a1, a2, a3, b[kk][2 * s], b[kk][2 * s + 1], 0.f, 0.f, 0.f, 0.f);
           else
@@ -753,7 +759,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) gemv_stream_kernel(const St
             const int step = 4 * word + i;
             if (word == 0 && i == 0)
               mma_first(acc[0], q[word] & mask, p[word] & mask, q8 & mask, p8 & mask, b[kk][0], b[kk][1],
-                        begin(0, 0), begin(0, 1), begin(0, 0), begin(0, 1));
+                        begin(0, 0), begin(0, 1), begin(0, 2), begin(0, 3));
             else if (word == 0)
               mma_first(acc[i], q[word] & mask, p[word] & mask, q8 & mask, p8 & mask, b[kk][2 * step], b[kk][2 * step + 1],
                         0.f, 0.f, 0.f, 0.f);
