@@ -105,10 +105,13 @@ def _(x, packed, scales, values, zeros, bias, outputs, group, bits, integer_grid
     return x.new_empty((x.shape[0], outputs))
 
 
+TILE_GEMM_DTYPES = (torch.float16, torch.bfloat16)
+
+
 def _plain(inputs: Tensor) -> bool:
     """Whether nothing but the values of ``inputs`` matters to an operation on it now."""
     return (type(inputs) in (Tensor, nn.Parameter) and not torch._C._functorch.is_functorch_wrapped_tensor(inputs)
-            and torch._C._len_torch_dispatch_stack() == 0 and not torch.jit.is_tracing()
+            and torch._C._len_torch_dispatch_stack() == 0 and not torch._C._is_tracing()
             and (forward_ad._current_level < 0 or forward_ad.unpack_dual(inputs).tangent is None)
             and not (torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") != inputs.dtype))
 
@@ -243,30 +246,9 @@ class PackedLinear(nn.Module):
             raise ValueError("packed inference requires CUDA inputs")
         rows = inputs.numel() // width
         if rows > self.maximum_fused_rows or rows == 0:
-            eager = (rows > 0 and self.layout is not None and not torch.compiler.is_compiling() and self._dense_weight is None
-                     and not (inputs.requires_grad and torch.is_grad_enabled()))
-            tiled = eager and self._takes_tile_gemm(inputs, rows)
-            chunked_rows = 2 * self.maximum_fused_rows if tiled else 4 * self.maximum_fused_rows
-            if eager and rows <= chunked_rows and inputs.dtype == torch.float16:
-                # a few rows more than one matvec takes: the matvec on chunks of eight rows streams the packed
-                # weight once per chunk, which measured faster than the tile GEMM up to 16 rows (16.5 against
-                # 19.5 us on 4096 -> 14336) and than reconstruct + library GEMM up to 32 rows for every codec
-                flat = inputs.reshape(rows, width).contiguous()
-                out = inputs.new_empty((rows, self.out_features))
-                plan = self._plan(inputs.dtype)
-                for start in range(0, rows, self.maximum_fused_rows):
-                    plan(flat[start:start + self.maximum_fused_rows], out[start:start + self.maximum_fused_rows])
-                return out.view(inputs.shape[:-1] + (self.out_features,))
-            if tiled:
-                # the weight is reconstructed inside the GEMM kernel, tile by tile
-                flat = inputs.reshape(rows, width).contiguous()
-                if flat.data_ptr() % 16:
-                    flat = flat.clone()
-                out = kernels.packed_tile_gemm(flat, self.packed, self.scales, self.values, self.zeros, self.bias,
-                                               inputs.new_empty((rows, self.out_features)), group=self.group,
-                                               bits=self.code_bits, integer_grid=self.integer_grid,
-                                               grid_minimum=self.grid_minimum)
-                return out.view(inputs.shape[:-1] + (self.out_features,))
+            out = None if torch.compiler.is_compiling() else self._many_rows(inputs, rows)
+            if out is not None:
+                return out
             return functional.linear(inputs, self.weight.to(inputs.dtype), self.bias)
         if inputs.requires_grad and torch.is_grad_enabled():
             raise RuntimeError("packed CUDA inference does not support autograd")
@@ -290,26 +272,62 @@ class PackedLinear(nn.Module):
                 out = self._plan(inputs.dtype)(flat, inputs.new_empty((rows, self.out_features)))
         return out.view(inputs.shape[:-1] + (self.out_features,))
 
-    def _takes_tile_gemm(self, inputs: Tensor, rows: int) -> bool:
-        dtype = inputs.dtype
-        if (self.packed.data_ptr() % 16 or self.in_features * self.code_bits // 8 % 16
-                or not kernels.tile_gemm_supported(rows, width=self.in_features, group=self.group, bits=self.code_bits,
-                                                   dtype=dtype, scales=self.scales, outputs=self.out_features)):
-            return False
-        form = dict(width=self.in_features, group=self.group, bits=self.code_bits, dtype=dtype, scales=self.scales,
-                    zeros=self.zeros, integer_grid=self.integer_grid, grid_minimum=self.grid_minimum,
-                    levels=self.values.numel())
-        if kernels.gemm_supported(rows, outputs=self.out_features, **form):
-            return True
-        # calls that would reconstruct and use functional.linear: what that sees and this launch does not stays there
-        # (tracers, functional transforms, tangents, autocast, a bias of another type), and a layer that keeps its
-        # reconstruction lets a call make it
-        if self.cache_dense or not _plain(inputs) or not (self.bias is None or self.bias.dtype == dtype):
-            return False
-        # small layers of a codec other than symmetric INT4 g128 in fp16: four matvec launches are as quick, and keep
-        # every row what the matvec gives for it alone
-        return (rows > 4 * self.maximum_fused_rows or dtype != torch.float16 or self.out_features * self.in_features >= 1 << 21
-                or kernels.gemm_supported(rows, **form))
+    def _many_rows(self, inputs: Tensor, rows: int) -> Tensor | None:
+        """More rows than one matvec takes, from the packed stream: matvec launches on chunks of rows, or the tile GEMM,
+        which reconstructs the weight inside the kernel; ``None`` where the dense weight and a library product serve.
+        The checks run on every eager call, which for a small layer lasts as long as its host side: cheap ones first."""
+        most = kernels.tile_gemm_rows(self.out_features, self.in_features, self.group, self.code_bits, self.integer_grid,
+                                      self._buffers["zeros"] is not None)
+        few = 4 * self.maximum_fused_rows
+        if (rows == 0 or (rows > most and rows > few) or self.layout is None
+                or (inputs.requires_grad and torch.is_grad_enabled())):
+            return None
+        buffers = self._buffers
+        if buffers["_dense_weight"] is not None:
+            return None
+        dtype, scales, zeros = inputs.dtype, buffers["scales"], buffers["zeros"]
+        tiled = (rows <= most and dtype in TILE_GEMM_DTYPES and scales.dtype == torch.float16
+                 and buffers["packed"].data_ptr() % 16 == 0)
+        if tiled and not (rows <= kernels.GEMM_MAXIMUM_ROWS and self._symmetric_int4(dtype, zeros)
+                          and (rows <= few or self.out_features * self.in_features >= 1 << 25)):
+            # calls that would reconstruct and use functional.linear: what that sees and this launch does not stays there
+            # (tracers, functional transforms, tangents, autocast, a bias of another type), and a layer that keeps its
+            # reconstruction lets a call make it
+            bias = buffers["bias"]
+            tiled = not self.cache_dense and _plain(inputs) and (bias is None or bias.dtype == dtype)
+        # The matvec on chunks of eight rows streams the packed weight once per chunk.  Up to 16 rows that measured faster
+        # than the tile GEMM (16.5 against 19.5 us on 4096 -> 14336), and up to 32 faster than reconstruct + library GEMM
+        # for every codec.  From 17 rows on the tile GEMM takes over, which rounds each weight to 16 bits, except where
+        # the matvec does not round it and the dense route of such rows never did (integer grids, one scale per 128
+        # codes), and for small layers, where four launches are as quick.
+        if rows <= few and dtype == torch.float16 and (
+                rows <= few // 2 or not tiled
+                or not (self._symmetric_int4(dtype, zeros)
+                        or (self.out_features * self.in_features >= 1 << 21
+                            and not (self.integer_grid and zeros is None and self.group % 128 == 0)))):
+            flat, out = self._flat(inputs, rows), inputs.new_empty((rows, self.out_features))
+            plan, step = self._plan(dtype), self.maximum_fused_rows
+            for start in range(0, rows, step):
+                plan(flat[start:start + step], out[start:start + step])
+        elif tiled:
+            flat, out = self._flat(inputs, rows), inputs.new_empty((rows, self.out_features))
+            if flat.data_ptr() % 16:
+                flat = flat.clone()
+            kernels.launch_tile_gemm(flat, buffers["packed"], scales, buffers["values"], zeros, buffers["bias"], out, rows,
+                                     self.out_features, self.in_features, self.group, self.code_bits, self.integer_grid,
+                                     self.grid_minimum)
+        else:
+            return None
+        return out if inputs.dim() == 2 else out.view(inputs.shape[:-1] + (self.out_features,))
+
+    def _flat(self, inputs: Tensor, rows: int) -> Tensor:
+        flat = inputs if inputs.dim() == 2 else inputs.reshape(rows, self.in_features)
+        return flat if flat.is_contiguous() else flat.contiguous()
+
+    def _symmetric_int4(self, dtype: torch.dtype, zeros: Tensor | None) -> bool:
+        """The form the first fused GEMM took: fp16 rows, the grid -8..7, one scale per 128 codes, no offsets."""
+        return (self.code_bits == 4 and self.group == 128 and dtype == torch.float16 and zeros is None and self.integer_grid
+                and self.grid_minimum == -8.0 and self._buffers["values"].numel() == 16)
 
     def extra_repr(self) -> str:
         return (f"in_features={self.in_features}, out_features={self.out_features}, bits={self.code_bits}, "

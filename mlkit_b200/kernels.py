@@ -6,6 +6,8 @@ on the current CUDA stream of the tensor's device, nothing is synchronised and, 
 output tensor the caller passes in, nothing is allocated.
 """
 
+import functools
+
 import torch
 from torch import Tensor
 
@@ -129,8 +131,8 @@ GEMM_MAXIMUM_ROWS = 128
 
 
 def gemm_workspace(device: torch.device, rows: int, outputs: int, width: int) -> Tensor:
-    """Zero-initialised scratch of the fused dequantise + GEMM kernel, one per (device, stream), grown to
-    the largest request; the kernel leaves it zeroed where it must be."""
+    """Scratch of ``mkb_gemm``, one per (device, stream), grown to the largest request: a zeroed head whose last word is
+    the status, then the partial sums."""
     need = _native.library().mkb_gemm_workspace_bytes(rows, outputs, width)
     if need <= 0:
         raise ValueError(f"no fused GEMM for {rows} rows, {outputs} outputs, width {width}")
@@ -158,10 +160,9 @@ def gemm_status() -> int:
 def gemm_supported(rows: int, *, width: int, group: int, bits: int, dtype: torch.dtype, scales: Tensor,
                    zeros: Tensor | None, integer_grid: bool, grid_minimum: float, levels: int,
                    outputs: int | None = None) -> bool:
-    """Whether ``packed_gemm`` covers the layer (the C entry point checks the same and more).  With
-    ``outputs`` given, also whether it is the faster route: measured on B200 against reconstruct +
-    library GEMM it wins at every shape up to 32 rows, and up to 128 rows once the weight has 2^25
-    codes (4096 x 8192) or more; small weights with many rows are quicker through the dense route."""
+    """Whether ``packed_gemm`` covers the layer (the C entry point checks the same and more).  With ``outputs`` given,
+    also whether it is a faster route than reconstruct + library GEMM whatever the layer: up to 32 rows, and up to 128
+    for weights of 2^25 codes or more.  (``tile_gemm_rows`` draws the finer line that ``PackedLinear`` follows.)"""
     if not (1 <= rows <= GEMM_MAXIMUM_ROWS and bits == 4 and group == 128 and width % 128 == 0 and zeros is None
             and dtype == torch.float16 and scales.dtype == torch.float16 and bool(integer_grid)
             and float(grid_minimum) == -8.0 and levels == 16):
@@ -171,7 +172,8 @@ def gemm_supported(rows: int, *, width: int, group: int, bits: int, dtype: torch
 
 def packed_gemm(x: Tensor, packed: Tensor, scales: Tensor, values: Tensor, bias: Tensor | None, out: Tensor, *,
                 group: int, bits: int, integer_grid: bool, grid_minimum: float) -> Tensor:
-    """``out[M, N] = x[M, K] @ dequant(packed)^T (+ bias)`` for up to 128 rows in one launch (``mkb_gemm``)."""
+    """``out[M, N] = x[M, K] @ dequant(packed)^T (+ bias)`` for up to 128 fp16 rows of symmetric INT4 (``mkb_gemm``): the
+    kernel of ``packed_tile_gemm`` with its partials in one workspace, for callers of the C ABI that own one."""
     device = _require_cuda(x, packed, scales, values, bias, out)
     rows, width = x.shape
     outputs = out.shape[1]
@@ -190,51 +192,88 @@ def packed_gemm(x: Tensor, packed: Tensor, scales: Tensor, values: Tensor, bias:
     return out
 
 
-def _status_word(device: torch.device) -> Tensor:
-    """The head whose last word is the status the tile GEMMs of a (device, stream) share."""
-    key = (device.index if device.index is not None else torch.cuda.current_device(),
-           torch.cuda.current_stream(device).cuda_stream)
-    held = _gemm_workspaces.get(key)
+def _status_pointer(device: torch.device, index: int, stream: int) -> int:
+    """The status word the tile GEMMs of a (device, stream) share: the last one of a workspace head."""
+    held = _gemm_workspaces.get((index, stream))
     if held is None:
-        held = _gemm_workspaces[key] = torch.zeros(1 << 20, dtype=torch.uint8, device=device)
-    return held
+        held = _gemm_workspaces[(index, stream)] = torch.zeros(1 << 20, dtype=torch.uint8, device=device)
+    return held.data_ptr() + 65532
 
 
-def tile_gemm_supported(rows: int, *, width: int, group: int, bits: int, dtype: torch.dtype, scales: Tensor,
-                        outputs: int) -> bool:
-    """Whether ``packed_tile_gemm`` covers a layer (the C entry point checks the same and more) and is the faster route.
-    Up to 128 rows it is ahead of reconstruct + library GEMM at every size measured (896 x 896 to 28672 x 4096).
-    Above, both multiply at the tensor cores' rate and what it saves is the reconstruction, so the weight has to be
-    large and the rows few: 4096 x 4096 at 1024 rows 42 us against 44, at 1537 rows 54 against 53; 1024 x 4096 at 512
-    rows 14.3 against 14.5, at 1024 rows 18 against 17."""
-    if not (2 <= bits <= 8 and group in (32, 64, 128) and width % 128 == 0 and dtype in (torch.float16, torch.bfloat16)
-            and scales.dtype == torch.float16):
-        return False
-    return rows <= 128 or (outputs * width >= 1 << 22 and rows <= 512) or (outputs * width >= 1 << 24 and rows <= 1024)
+# Most rows for which the tile GEMM was not slower than reconstruct + library GEMM, measured on B200 over 32 shapes from
+# 128 x 896 to 28672 x 4096, every codec, fp16 and bf16 (device time, weights cold in L2).  Both multiply at the tensor
+# cores' rate; the tile GEMM saves writing the weight and reading it back, and pays its decode once per tile of up to 256
+# rows, so the line moves up with the weight's size and down with the cost of the decode.  In us, tile / dense: 4 bits with
+# offsets, 4096 x 4096, 768 rows 36.9 / 39.1, 1024 rows 45.3 / 43.9; 4 bits, 4864 x 896, 160 rows 10.8 / 11.2, 512 rows
+# 15.1 / 11.8; 8 bits, 4096 x 4096, 128 rows 19.7 / 26.1, 1024 rows 85.6 / 42.3.
+# By the width of the layer: (codes of the weight, most rows of: 4-bit integer grids; those with offsets; other codecs of up
+# to 5 bits; 6 bits; 7 and 8 bits), the last line whose codes the weight reaches.  0: one tile of rows, the most of its
+# decode.
+_MI = 1 << 20
+_TILE_ROWS = (
+    (1024, ((0, (48, 48, 48, 48, 48)), (_MI, (96, 96, 96, 96, 64)), (4 * _MI, (160, 160, 160, 160, 64)))),
+    (2048, ((0, (48, 48, 48, 48, 48)), (_MI, (128, 128, 96, 128, 128)), (2 * _MI, (160, 160, 160, 160, 128)),
+            (3 * _MI, (192, 192, 192, 192, 0)), (8 * _MI, (448, 320, 224, 224, 0)), (16 * _MI, (1024, 1024, 448, 384, 0)))),
+    (1 << 30, ((0, (48, 48, 48, 48, 48)), (_MI, (128, 128, 128, 128, 128)), (3 * _MI // 2, (160, 160, 160, 160, 128)),
+               (2 * _MI, (256, 256, 192, 224, 192)), (3 * _MI, (384, 320, 192, 320, 192)), (4 * _MI, (384, 384, 192, 384, 192)),
+               (6 * _MI, (448, 448, 224, 320, 0)), (8 * _MI, (448, 448, 256, 320, 0)), (9 * _MI, (896, 768, 448, 448, 0)),
+               (24 * _MI, (1024, 1024, 640, 448, 0)), (56 * _MI, (1024, 1024, 768, 512, 256)))),
+)
+
+
+@functools.lru_cache(maxsize=4096)
+def tile_gemm_rows(outputs: int, width: int, group: int, bits: int, integer_grid: bool, offsets: bool = False) -> int:
+    """Most activation rows (fp16 or bf16) of a layer that ``packed_tile_gemm`` is the faster route for; 0 where it does
+    not cover the layer (the C entry point checks the same and more)."""
+    if not (2 <= bits <= 8 and group in (32, 64, 128) and width % 128 == 0 and width * bits // 8 % 16 == 0):
+        return 0
+    decoder = (1 if offsets else 0) if bits == 4 and integer_grid else 2 if bits <= 5 else 3 if bits == 6 else 4
+    lines = next(lines for below, lines in _TILE_ROWS if width < below)
+    rows = next(rows for codes, rows in reversed(lines) if outputs * width >= codes)[decoder]
+    return rows or (176 if bits == 7 else 160) - (16 if offsets else 0)     # the tiles shared memory leaves room for
+
+
+@functools.lru_cache(maxsize=64)
+def _partial_bytes(rows: int, index: int) -> int:
+    return _native.library().mkb_gemm_tile_partial_bytes(rows)
 
 
 def packed_tile_gemm(x: Tensor, packed: Tensor, scales: Tensor, values: Tensor, zeros: Tensor | None, bias: Tensor | None,
                      out: Tensor, *, group: int, bits: int, integer_grid: bool, grid_minimum: float) -> Tensor:
     """``out[M, N] = x[M, K] @ dequant(packed)^T (+ bias)`` for any number of rows (``mkb_gemm_tile``); the weight is
     rounded to the type of ``x`` and never written to memory."""
-    device = _require_cuda(x, packed, scales, values, zeros, bias, out)
+    _require_cuda(x, packed, scales, values, zeros, bias, out)
     rows, width = x.shape
     if not x.is_contiguous() or not out.is_contiguous() or out.dtype != x.dtype or out.shape[0] != rows:
         raise ValueError("packed_tile_gemm needs contiguous activations and outputs of one type and number of rows")
     if zeros is not None and zeros.dtype != scales.dtype:
         raise ValueError("offsets must share the dtype of the scales")
+    launch_tile_gemm(x, packed, scales, values, zeros, bias, out, rows, out.shape[1], width, group, bits, integer_grid,
+                     grid_minimum)
+    return out
+
+
+def launch_tile_gemm(x: Tensor, packed: Tensor, scales: Tensor, values: Tensor, zeros: Tensor | None, bias: Tensor | None,
+                     out: Tensor, rows: int, outputs: int, width: int, group: int, bits: int, integer_grid: bool,
+                     grid_minimum: float) -> None:
+    """``packed_tile_gemm`` of tensors a caller answers for: one device, contiguous, offsets of the scales' type."""
+    index = x.get_device()
+    if torch.cuda.current_device() != index:
+        with torch.cuda.device(index):
+            return launch_tile_gemm(x, packed, scales, values, zeros, bias, out, rows, outputs, width, group, bits,
+                                    integer_grid, grid_minimum)
     if bias is not None and bias.dtype != x.dtype:
         bias = bias.to(x.dtype)
-    library = _native.library()
-    with torch.cuda.device(device):
-        partials = torch.empty(library.mkb_gemm_tile_partial_bytes(rows), dtype=torch.uint8, device=device)
-        status = library.mkb_gemm_tile(
-            x.data_ptr(), packed.data_ptr(), scales.data_ptr(), values.data_ptr(), _pointer(zeros), _pointer(bias), out.data_ptr(),
-            rows, out.shape[1], width, group, bits, values.numel(), _tag(x.dtype, "activation"), _tag(scales.dtype, "scale"),
-            width * bits // 8, scales.stride(0) if scales.dim() == 2 else -(-width // group), int(integer_grid),
-            float(grid_minimum), partials.data_ptr(), partials.numel(), _status_word(device).data_ptr() + 65532, _stream(device))
-    _native.check(status, "packed_tile_gemm")
-    return out
+    stream = torch.cuda.current_stream().cuda_stream
+    size = _partial_bytes(rows, index)
+    partials = x.new_empty(size, dtype=torch.uint8)
+    status = _native.library().mkb_gemm_tile(
+        x.data_ptr(), packed.data_ptr(), scales.data_ptr(), values.data_ptr(), _pointer(zeros), _pointer(bias), out.data_ptr(),
+        rows, outputs, width, group, bits, values.numel(), _tag(x.dtype, "activation"), _tag(scales.dtype, "scale"),
+        width * bits // 8, scales.stride(0) if scales.dim() == 2 else -(-width // group), int(integer_grid),
+        float(grid_minimum), partials.data_ptr(), size, _status_pointer(x.device, index, stream), stream)
+    if status:
+        _native.check(status, "packed_tile_gemm")
 
 
 def packed_matvec(x: Tensor, packed: Tensor, scales: Tensor, values: Tensor, zeros: Tensor | None,

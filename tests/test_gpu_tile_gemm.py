@@ -143,3 +143,17 @@ def test_calls_that_see_more_than_values_keep_the_dense_route():
     assert module(x.requires_grad_()).requires_grad
     with pytest.raises(RuntimeError):       # a bias of another type
         packed_linear(1024, 4096, torch.float32, bias=True)(x.detach())
+
+
+@pytest.mark.parametrize("bits", [2, 3, 5, 6, 7, 8])
+def test_few_rows_of_integer_grids_keep_what_the_matvec_gives(bits):
+    """17 to 32 fp16 rows of these grids run as matvec launches, which round no weight: every row is, bit for bit, what
+    the matvec gives for it."""
+    import mlkit_b200 as mk
+
+    torch.manual_seed(bits)
+    linear = torch.nn.Linear(2048, 2048, device="cuda", dtype=torch.float16)
+    module = mk.PackedLinear(linear, mk.int(bits)(linear.weight.detach().float(), mk.Ctx("layer", device="cuda")))
+    x = torch.randn(32, 2048, device="cuda").half()
+    for rows in (17, 24, 32):
+        assert torch.equal(module(x[:rows]), torch.cat([module(part) for part in x[:rows].split(8)]))

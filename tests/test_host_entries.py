@@ -49,3 +49,24 @@ def test_bounded_waits_of_the_tile_gemm_end_for_whole_warps():
     assert deciding == ["__device__ __forceinline__ bool tile_wait(uint64_t* bar, uint32_t parity, volatile int* failed) {",
                         "return __all_sync(0xffffffffu, tile_wait(bar, parity, failed));"]
     assert "__all_sync(0xffffffffu, tile_wait" in source and source.count("tile_wait_warp(") > 5
+
+
+def test_tile_gemm_covers_what_its_rule_admits():
+    for bits in range(1, 9):
+        for group in (16, 32, 64, 96, 128, 256):
+            for width in (64, 128, 192, 256, 896, 1000, 4096):
+                status = _native.library().mkb_gemm_tile(
+                    POINTER, POINTER, POINTER, POINTER, None, None, POINTER, 33, 64, width, group, bits, 1 << bits, F16, F16,
+                    width * bits // 8, -(-width // group), 1, -float(1 << bits - 1), POINTER, 1 << 40, POINTER, None)
+                admitted = kernels.tile_gemm_rows(64, width, group, bits, True) > 0
+                assert (status != UNSUPPORTED) == admitted, (bits, group, width)
+
+
+def test_tile_gemm_takes_more_rows_of_larger_weights():
+    for bits in range(2, 7):
+        for integer in (True, False):
+            for width in (896, 1024, 4096, 14336):
+                most = [kernels.tile_gemm_rows(outputs, width, 128, bits, integer) for outputs in (64, 512, 2048, 8192, 28672)]
+                assert most == sorted(most) and 32 < most[0] <= most[-1] <= 1024
+    # eight bits decode slowest: two tiles of rows cost more than writing the weight once
+    assert kernels.tile_gemm_rows(4096, 4096, 128, 8, True) < kernels.tile_gemm_rows(4096, 4096, 128, 4, True)
