@@ -48,7 +48,9 @@ enum {
   MKB_GEMV_BULK = 4,   /* TMA-fed kernel: whole 16-row units by cp.async.bulk.tensor into a shared-memory ring
                           (INT4 integer grid, fp16, K % 256 == 0; needs the workspace when K is split) */
   MKB_GEMV_STREAM = 5  /* streaming kernel: activations in registers, weights through per-warp cp.async rings
-                          (integer grid, fp16, group 128, K % 128 == 0); what AUTO takes when it applies */
+                          (K % 128 == 0; by name: fp16 without offsets, integer grids with group 128, 4-bit ones
+                          and tables of at most 16 levels with 64 or 128).  What AUTO takes when it applies, and
+                          AUTO also takes it for bf16, and for 4-bit integer grids with offsets or group 32 */
 };
 
 int mkb_version(void);
@@ -153,8 +155,8 @@ int mkb_gemv_static_status(int* status);
  * the result equals mkb_hadamard followed by mkb_gemv bit for bit; no rotated activation is written to
  * or read from global memory.
  * signs: int8 [K] of +1 / -1, 16-byte aligned, or null for the plain transform.
- * Covers what the streaming matvec covers (fp16 activations and scales; INT2/4/8 on the integer grid with
- * groups of 128, 3- and 4-bit tables with groups of 64 or 128) when K is a power of two >= 512 and
+ * Covers what MKB_GEMV_STREAM covers by name (fp16 activations and scales; integer grids of 2 to 8 bits with
+ * groups of 128, 3- and 4-bit codes with groups of 64 or 128; no bf16, no offsets) when K is a power of two >= 512 and
  * M * K * 4 <= 65536 (K = 4096: M <= 4); anything else returns MKB_E_UNSUPPORTED and the caller runs
  * mkb_hadamard, then mkb_gemv.  Widths with an odd factor (14336 = 28 * 512) are not covered.
  */
@@ -260,7 +262,8 @@ int mkb_rtn_encode(const void* weight, const float* levels, uint8_t* packed, voi
  * group in the same shape when `offsets` is not null (asymmetric formats: w = level * scale + offset), and with
  * *nonfinite (device) set to 0, or to 1 when a weight is infinite or NaN (the outputs are then meaningless).
  * `levels` may be null for integer grids.
- * Covers groups of 8 to 256 codes (a power of two), K % 8 == 0 and a 16-byte aligned weight;
+ * Covers groups of 8 to 256 codes (a power of two), K % 8 == 0, a 16-byte aligned weight and 8-byte aligned packed
+ * and codes_out;
  * everything else is MKB_E_UNSUPPORTED. */
 int mkb_rtn_encode_checked(const void* weight, const float* levels, uint8_t* packed, float* scales, float* offsets,
                            uint8_t* codes_out, int* nonfinite, int64_t N, int K, int group, int bits, int level_count,

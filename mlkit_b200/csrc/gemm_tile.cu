@@ -2,7 +2,8 @@
 // takes, any codec of 2 to 8 bits, fp16 or bf16 activations (sm_100a).
 //
 // The weight is read as codes; reconstructed 16-bit weights exist in shared memory only.  A tile of the result is 128
-// weight rows (the M of tcgen05.mma) x up to 240 activation rows (its N), fp32 in tensor memory.  A stage of the pipeline
+// weight rows (the M of tcgen05.mma) x up to 256 activation rows (its N; what shared memory leaves: 256 at 2 bits, 224 for
+// 4-bit integer grids, 208 with offsets, 160 at 8 bits, 144 with offsets), fp32 in tensor memory.  A stage of the pipeline
 // is a block of 128 K: 32 KB of weights and 256 B per activation row, as two K-major halves in the 128-byte swizzle.
 // Roles (23 warps):
 //   * warps 0-15 decode, two groups of eight, a block each in turn: a block is a chain of waits, loads and stores, and
@@ -21,9 +22,10 @@
 // partial, and a second, dependent launch adds the partials of every cut tile in K order on all SMs.
 // All hand-offs inside the CTA are mbarriers with bounded waits: on expiry the CTA records a status word and drains.
 //
-// 4096 -> 14336 in 4 bits, fp16 rows, against reconstruct + library GEMM: 16 rows 19.5 (82), 64 rows 23.6 (84), 128 rows
-// 27 (85), 512 rows 67 (111), 1024 rows 118 us (147).  Up to 64 rows the decode bounds it (about 450 cycles per block),
-// above 200 the activations' traffic from L2 and the tensor core.
+// 4096 -> 14336 in 4 bits, fp16 rows, us (against reconstruct + library GEMM): 17 rows 19.5 (81), 64 rows 23.3 (84), 128
+// rows 26.8 (84), 512 rows 67 (109), 1024 rows 120 (146).  Above 200 rows the activations' traffic from L2 and the tensor
+// core bound it.  Up to 64 rows neither does, nor the codes' 4.6 us from HBM: an SM has 25 blocks, whose decode takes about
+// 450 cycles each (5.7 us in all), so most of the launch pair's time there is its start, its pipeline's and its sums'.
 #include <cuda.h>
 
 #include <algorithm>
