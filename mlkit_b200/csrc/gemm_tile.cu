@@ -91,10 +91,12 @@ __device__ __forceinline__ bool tile_wait(uint64_t* bar, uint32_t parity, volati
   *failed = 1;
   return false;
 }
-// The same by a whole warp: either every lane goes on or none does.  A lane that left alone would stand at the closing
-// barrier of the CTA while the others wait for it at their next warp barrier.
-__device__ __forceinline__ bool tile_wait_warp(uint64_t* bar, uint32_t parity, volatile int* failed) {
-  return __all_sync(0xffffffffu, tile_wait(bar, parity, failed));
+// The same for copies in flight after a failure: their stage may also miss decoders, so this one only gives them time.
+__device__ __forceinline__ void tile_drain(uint64_t* bar, uint32_t parity) {
+  uint32_t done = 0;
+  for (int spins = 0; spins < 64 && !done; ++spins)
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+                 : "=r"(done) : "r"(tile_shared(bar)), "r"(parity), "r"(20000u) : "memory");
 }
 // The warps that issue products and copies run whole: every lane holds the same values, which the compiler keeps in
 // uniform registers, where these instructions take their operands from, and one elected lane issues.  (With one lane
@@ -261,8 +263,9 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_tile_kernel(const __grid
     const uint32_t row_at = tile_shared(weight_s) + h * kWeightHalf + r * 128 + ((r & 7) << 4);
     int stage = group % a.stages, round = group / a.stages;
     uint32_t code_slot = group, code_round = 0, slot = 0;      // (at least four code slots)
-    for (int i = group; i < count; i += kDecodeGroups) {
-      if (!tile_wait_warp(&bars.codes_full[code_slot], code_round & 1u, failed)) break;
+    int i = group;
+    for (; i < count; i += kDecodeGroups) {
+      if (!tile_wait(&bars.codes_full[code_slot], code_round & 1u, failed)) break;
       uint32_t words[WORDS];
       const uint32_t row_from = tile_shared(code_s) + code_slot * CODE_SLOT + r * (16 * BITS);
 #pragma unroll
@@ -299,7 +302,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_tile_kernel(const __grid
       if (a.zeros != nullptr) side(kDecodeThreads * 8, zeros);
       slot = slot + 1 == kScaleSlots ? 0 : slot + 1;
       copy_scales();                   // into the slot read one block ago
-      if (round > 0 && !tile_wait_warp(&bars.stage_empty[stage], uint32_t(round - 1) & 1u, failed)) break;
+      if (round > 0 && !tile_wait(&bars.stage_empty[stage], uint32_t(round - 1) & 1u, failed)) break;
       const uint32_t to = row_at + 2 * stage * kWeightHalf;
 #pragma unroll
       for (int c = 0; c < 8; ++c) {    // chunks of eight codes
@@ -357,6 +360,10 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_tile_kernel(const __grid
       stage += kDecodeGroups;
       if (stage >= a.stages) { stage -= a.stages; ++round; }
     }
+    // A lane whose wait gave up has left the loop alone: it meets the others at the warp barriers of the blocks that it
+    // leaves out, or they would stand there while it stands at the CTA's closing barrier.  (Leaving by a vote per block, or
+    // staying in the loop without waiting, made 64 rows 1 % slower.)
+    for (; i < count; i += kDecodeGroups) __syncwarp();
     asm volatile("cp.async.wait_group 0;" ::: "memory");
   } else if (warp < 20) {
     // ================================ epilogue ================================
@@ -369,7 +376,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_tile_kernel(const __grid
       const bool whole = unit == tile_begin && stop == tile_end;
       const int row_block = tile / a.column_tiles, m0 = (tile - row_block * a.column_tiles) * a.columns;
       const int live = min(a.columns, a.M - m0), n = row_block * kTileRows + row;
-      const bool good = tile_wait_warp(&bars.sums_full[buffer], uint32_t(uses) & 1u, failed);
+      const bool good = tile_wait(&bars.sums_full[buffer], uint32_t(uses) & 1u, failed);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const float bias = a.bias == nullptr || n >= a.N ? 0.f
                          : BF16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(a.bias)[n])
@@ -423,7 +430,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_tile_kernel(const __grid
     const int tile = first / a.k_blocks;
     int m0 = (tile % a.column_tiles) * a.columns, block = first - tile * a.k_blocks, stage = 0, round = 0, sent = 0;
     for (int i = 0; i < count; ++i) {
-      if (round > 0 && !tile_wait_warp(&bars.stage_empty[stage], uint32_t(round - 1) & 1u, failed)) break;
+      if (round > 0 && !__all_sync(0xffffffffu, tile_wait(&bars.stage_empty[stage], uint32_t(round - 1) & 1u, failed))) break;
       const uint32_t bar = tile_shared(&bars.stage_full[stage]), to = tile_shared(rows_s) + 2 * stage * rows_half;
       asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
                    "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%4], %5;\n\t"
@@ -440,10 +447,9 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_tile_kernel(const __grid
       }
       if (++stage == a.stages) { stage = 0; ++round; }
     }
-    // no copy is left in flight when the CTA ends.  (After a failure elsewhere a stage may also miss decoders: then the
-    // wait only gives the copy time.)
-    for (int i = max(0, sent - a.stages); i < sent; ++i)
-      tile_wait(&bars.stage_full[i % a.stages], uint32_t(i / a.stages) & 1u, failed);
+    // no copy is left in flight when the CTA ends, whatever happened to its consumers
+    for (int i = max(0, sent - a.stages); *failed && i < sent; ++i)
+      tile_drain(&bars.stage_full[i % a.stages], uint32_t(i / a.stages) & 1u);
   } else if (warp == 22) {
     // ================================ codes ================================
     const uint64_t map = reinterpret_cast<uint64_t>(&codes_map);
@@ -451,7 +457,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_tile_kernel(const __grid
     int block = first - tile * a.k_blocks, m0 = (tile - row_block * a.column_tiles) * a.columns, rows = row_block * kTileRows;
     int slot = 0, round = 0, sent = 0;
     for (int i = 0; i < count; ++i) {
-      if (round > 0 && !tile_wait_warp(&bars.codes_empty[slot], uint32_t(round - 1) & 1u, failed)) break;
+      if (round > 0 && !__all_sync(0xffffffffu, tile_wait(&bars.codes_empty[slot], uint32_t(round - 1) & 1u, failed))) break;
       asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
                    "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%4], %5;\n\t"
                    "@q cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n\t}\n"
@@ -476,11 +482,11 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_tile_kernel(const __grid
     bool alive = true;
     while (unit < end && alive) {
       const int stop = min((unit / a.k_blocks + 1) * a.k_blocks, end);
-      if (uses > 0 && !tile_wait_warp(&bars.sums_empty[buffer], uint32_t(uses - 1) & 1u, failed)) break;
+      if (uses > 0 && !__all_sync(0xffffffffu, tile_wait(&bars.sums_empty[buffer], uint32_t(uses - 1) & 1u, failed))) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t sums = tmem + buffer * (a.tmem_columns >> 1);
       for (int i = 0; i < stop - unit; ++i) {
-        if (!tile_wait_warp(&bars.stage_full[stage], uint32_t(round) & 1u, failed)) { alive = false; break; }
+        if (!__all_sync(0xffffffffu, tile_wait(&bars.stage_full[stage], uint32_t(round) & 1u, failed))) { alive = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint64_t weights = tile_descriptor(tile_shared(weight_s) + 2 * stage * kWeightHalf);
         const uint64_t rows = tile_descriptor(tile_shared(rows_s) + 2 * stage * rows_half);

@@ -1,7 +1,6 @@
 """What the C entry points accept and refuse, on the host alone.  The pointers are addresses that nothing may read, so
 these tests do not run where a device would: there the calls that are accepted would launch."""
 
-import re
 from pathlib import Path
 
 import pytest
@@ -40,15 +39,18 @@ def test_many_row_transform_covers_what_its_rule_admits():
                 assert (status != UNSUPPORTED) == admitted, (factor, power, dtype)
 
 
-def test_bounded_waits_of_the_tile_gemm_end_for_whole_warps():
-    """By reading the source, an expired wait being nothing to bring about on a device: wherever the outcome of a wait
-    decides what its lanes do next it is voted on by the warp, and what is left of the plain wait only waits."""
+def test_lanes_whose_wait_expired_keep_their_warp_barriers():
+    """By reading the source, an expired wait being nothing to bring about on a device.  The decoders' loop has one warp
+    barrier per block, behind both waits, and a lane that left at a wait meets the others at the barriers it leaves out;
+    every other wait that ends a loop is voted on by the warp."""
     source = (Path(kernels.__file__).parent / "csrc" / "gemm_tile.cu").read_text()
-    uses = [line.strip() for line in source.splitlines() if re.search(r"\btile_wait\(", line)]
-    deciding = [line for line in uses if not line.startswith("tile_wait(")]
-    assert deciding == ["__device__ __forceinline__ bool tile_wait(uint64_t* bar, uint32_t parity, volatile int* failed) {",
-                        "return __all_sync(0xffffffffu, tile_wait(bar, parity, failed));"]
-    assert "__all_sync(0xffffffffu, tile_wait" in source and source.count("tile_wait_warp(") > 5
+    step = "i < count; i += kDecodeGroups)"
+    decoders = source[source.index(step):source.index("// ================================ epilogue")]
+    loop, left = decoders.split("for (; " + step)
+    assert loop.count("__syncwarp();") == 1 and left.lstrip().startswith("__syncwarp();")
+    assert loop.count("tile_wait(") == 2 and loop.rindex("tile_wait(") < loop.index("__syncwarp();") and loop.count("break;") == 2
+    for line in source[source.index("// ================================ epilogue"):].splitlines():
+        assert "tile_wait(" not in line or "__all_sync(0xffffffffu, tile_wait(" in line or "break" not in line
 
 
 def test_tile_gemm_covers_what_its_rule_admits():
