@@ -445,9 +445,9 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) gemv_stream_kernel(const St
   // RAW: sum(x) * 2^-24 of a k-tile's scale group for activation rows 2t, 2t + 1; without offsets already times
   // the grid minimum, which makes it the accumulators' start.  With one group it is held twice, as the four registers
   // in a row that a tensor-core step starts from: put together in the loop they cost the plain matvec 1-2 % (8 rows of
-  // 4096 -> 6144: 5.53 us against 5.40).  3 and 8 bits are short of registers and, like single k-tiles per visit,
-  // quicker with pairs.
-  constexpr int STARTS = V::SUMS == 1 && !ZERO && KT == 2 && BITS != 3 && BITS != 8 ? 4 : 2;
+  // 4096 -> 6144: 5.53 us against 5.40).  What is short of registers, 3 and 8 bits and with bf16 everything
+  // above four bits, is quicker with pairs, like single k-tiles per visit.
+  constexpr int STARTS = V::SUMS == 1 && !ZERO && KT == 2 && (BITS == 2 || BITS == 4 || (!BF && BITS != 3 && BITS != 8)) ? 4 : 2;
   float start[KT][V::SUMS][STARTS];
   [[maybe_unused]] float down[2] = {1.f, 1.f};   // bf16: what moves the sums of activation rows 2t, 2t + 1 back
   [[maybe_unused]] bool unbounded = false;       // bf16: row g has an infinity or a NaN in this warp's slice
@@ -947,7 +947,9 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) gemv_stream_kernel(const St
     if (visit0 + R - batch_first < a.batch && visit0 + R < a.visits) continue;
 
     // ---- end of a batch: add the warps' partial sums in warp order, four outputs per thread ----
-    if constexpr (REDO) redo = __syncthreads_or(redo_rows() != 0);
+    // (whether a row is to be redone travels with this barrier; with bf16 it is asked after the last reduction, where eight
+    // bits, out of registers, take it better: a head of 128256 x 4096 at three rows 97 us against 103)
+    if constexpr (REDO && !BF) redo = __syncthreads_or(redo_rows() != 0);
     else __syncthreads();
     const int in_batch = min(a.batch, a.visits - batch_first);
     const int quads = in_batch * a.RG * 32;
@@ -1003,6 +1005,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) gemv_stream_kernel(const St
   // ---- rows with an infinity or a NaN: plain products over the whole row, one warp per output.  The CTAs of a
   // cluster that saw one write the same values, after the barrier above ----
   if constexpr (REDO) {
+    if constexpr (BF) redo = __syncthreads_or(unbounded);
     if (redo) {
       auto activation = [&](int m, int k) -> float {
         const int64_t at = int64_t(m) * (GATED ? 2 * a.K : a.K) + k;
